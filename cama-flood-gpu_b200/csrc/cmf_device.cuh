@@ -87,6 +87,10 @@ constexpr int kCtlMaxSteps = 1;   // max over members of the sub-step count
 constexpr int kCtlBlocksDone = 2; // last-block-done counter of k_stage
 constexpr int kCtlBarrier = 4;    // [4..5]: arrival counter (u64) of the persistent kernel's grid barrier
 constexpr int kCtlAbort = 6;      // set when a grid barrier gave up: every block leaves the interval
+constexpr int kCtlCflMax = 8;     // resident kernel: CFL sub-step count, maximum over the tiles
+constexpr int kCtlEpoch = 9;      // resident kernel: last epoch of the exchanged values
+constexpr int kCtlTileMax = 10;   // [10..14]: TileCounts of the resident kernel
+constexpr int kResidentMaxTiles = 256;  // flags of the resident kernel (cmf_resident.cuh)
 constexpr int kHardSubStepCap = 100000;  // bound of the device-side sub-step loop
 
 // Two fluxes of one element stored together (river, floodplain): one 8-byte
@@ -144,6 +148,10 @@ struct Dev {
     int* nsub;
     int* cur;
     int* ctl;
+    // resident kernel (null where the plan has none): flags of its tiles and
+    // the values they exchange
+    unsigned* rflag;
+    unsigned long long *xflux, *xeta, *xrate, *xend, *xsum, *xprate;
     double* tsec;  // outer interval in seconds (double)
     double* budget;
     double* bpart;  // [kBudgetTerms][cell_blocks]
@@ -266,11 +274,136 @@ __device__ __forceinline__ StepInfo step_info(const int* ctl, const int* nsub, i
 }
 
 // ---------------------------------------------------------------------------
-// k_momentum, cell part: a catchment's outflow over the sub-step
+// Cell part of the momentum phase: a catchment's outflow over the sub-step
 // (outflow.cu:21-175, reservoir.cu:18-94), from the physics of
-// cmf_physics.cuh.  Writes the unlimited river and floodplain fluxes and the
-// new interface state (flow depths, floodplain flow area).
+// cmf_physics.cuh: the unlimited river and floodplain fluxes and the new
+// interface state (flow depths, floodplain flow area).  k_momentum takes the
+// cell's fields from the model tensors, the resident kernel from a tile in
+// shared memory; what only some cells need comes through `rare`.
 // ---------------------------------------------------------------------------
+template <typename REAL>
+struct MomentumCell {
+    REAL width, len, bank_h, n_riv, n_fld, elev, dx;
+    REAL q_riv, q_fld;              // fluxes of the last sub-step
+    REAL h_riv, h_fld;              // depths
+    REAL hr_before, hf_before, af_before;  // interface state of the last sub-step
+    REAL s_fld;                     // flood storage
+    REAL elev_dn, eta_dn;           // downstream elevation and water surface (the sea's at a mouth)
+};
+
+template <typename REAL>
+struct MomentumRates {
+    REAL q_riv, q_fld;         // unlimited fluxes
+    REAL h_riv, h_fld, a_fld;  // interface flow depths, floodplain flow area
+    REAL eta;                  // water surface of the cell
+};
+
+template <typename REAL, bool RES, bool LEV, typename Rare>
+__device__ __forceinline__ MomentumRates<REAL> momentum_rates(const MomentumCell<REAL>& c, uint8_t fl, REAL dt,
+                                                              REAL g, REAL min_kin, const Rare& rare)
+{
+    const REAL gdt = g * dt;
+    const bool mouth = fl & CMF_CELL_MOUTH;
+    const bool lev_cell = LEV && (fl & CMF_CELL_LEVEE);
+    const bool res_cell = RES && (fl & CMF_CELL_RESERVOIR);
+
+    // water surfaces: this cell's over its river bed; downstream the next
+    // cell's, or the sea at this catchment's elevation for a mouth
+    const REAL bed = c.elev - c.bank_h;
+    const REAL eta = c.h_riv + bed;
+    const REAL eta_top = smax(eta, c.eta_dn);
+    const REAL slope = (eta - c.eta_dn) / c.dx;
+
+    // interface state: river flow depth (the own depth at a mouth, whose sea
+    // level sets the slope only), floodplain flow depth and flow area
+    const REAL hr_now = mouth ? c.h_riv : eta_top - bed;
+    const REAL hf_now = smax((mouth ? eta : eta_top) - c.elev, REAL(0));
+    const REAL af_now = smax(c.s_fld / c.len - c.h_fld * c.width, REAL(0));
+    const REAL hr_si = implicit_mean(hr_now, c.hr_before, REAL(1e-6));
+    const REAL hf_si = implicit_mean(hf_now, c.hf_before, REAL(1e-6));
+
+    REAL q_riv = REAL(0);
+    if (hr_si > REAL(1e-5) && hr_now * c.width > REAL(1e-5))
+        q_riv = channel_discharge(c.q_riv, c.width, c.n_riv, hr_si, slope, gdt);
+    REAL q_fld = REAL(0);
+    if (hf_si > REAL(1e-5) && af_now > REAL(1e-5)) {
+        const REAL af_si = implicit_mean(af_now, smax(c.af_before, REAL(1e-6)), REAL(1e-6));
+        q_fld = plain_discharge(c.q_fld, af_si, c.n_fld, hf_si, capped_slope(slope, REAL(0.005)), gdt);
+    }
+    // the floodplain never flows against the river
+    if (q_riv * q_fld < REAL(0)) q_fld = REAL(0);
+
+    // river storage, read only where a rule below needs it
+    REAL s_riv = REAL(0);
+    bool have_s_riv = false;
+    auto river_store = [&]() -> REAL {
+        if (!have_s_riv) {
+            s_riv = rare.river_store();
+            have_s_riv = true;
+        }
+        return s_riv;
+    };
+    // backwater into the cell draws at most 5 % of what it holds per sub-step
+    if (q_riv < REAL(0) && !mouth) {
+        const REAL held = river_store() + c.s_fld + (lev_cell ? rare.protected_store() : REAL(0));
+        const REAL rate = smin(REAL(0.05) * held / ((-q_riv - q_fld) * dt), REAL(1));
+        q_riv *= rate;
+        q_fld *= rate;
+    }
+    if (RES && (fl & CMF_CELL_DAM_UPSTREAM)) {
+        const REAL bed_slope = smax((c.elev - c.elev_dn) / c.dx, min_kin);
+        kinematic_outflow(bed_slope, c.len, c.h_riv, c.h_fld, river_store(), c.s_fld, c.width, c.n_riv,
+                          c.n_fld, dt, q_riv, q_fld);
+    }
+    if (res_cell) {
+        // the release replaces the routed flux; the limiter gathers fluxes,
+        // so nothing scattered before needs undoing
+        q_riv = dam_release(rare.dam_rule(), river_store() + c.s_fld, rare.dam_inflow(), dt);
+        q_fld = REAL(0);
+    }
+    return {q_riv, q_fld, hr_now, hf_now, af_now, eta};
+}
+
+// Diagnostics of the momentum phase, on the member's last sub-step.
+template <typename REAL, bool RES, bool LEV, typename Rare>
+__device__ __forceinline__ void momentum_diagnostics(const Dev<REAL>& v, REAL elev, REAL s_fld, uint8_t fl, long im,
+                                                     REAL eta, const Rare& rare)
+{
+    const bool lev_cell = LEV && (fl & CMF_CELL_LEVEE);
+    const bool res_cell = RES && (fl & CMF_CELL_RESERVOIR);
+    if (v.wse) v.wse[im] = eta;
+    if (v.pwse) v.pwse[im] = lev_cell ? smin(elev + rare.protected_depth(), eta) : eta;
+    if (v.tsto) {
+        const REAL held = res_cell ? rare.river_store() + s_fld
+                                   : rare.river_store() + s_fld + (lev_cell ? rare.protected_store() : REAL(0));
+        v.tsto[im] = (double)held;
+    }
+}
+
+template <typename REAL>
+__device__ __forceinline__ DamRule<REAL> dam_rule_of(const Dev<REAL>& v, long i)
+{
+    const int slot = v.rslot[i];
+    return {v.rcons[slot], v.radj[slot], v.remerg[slot], v.rnout[slot], v.raout[slot], v.rfcout[slot]};
+}
+
+// The rarely read fields of a cell, in the model tensors.
+template <typename REAL, bool ONE>
+struct GlobalRare {
+    const Dev<REAL>& v;
+    const double* __restrict__ rsrc;  // river storage before the sub-step
+    long i, im;
+    int m;
+    __device__ REAL river_store() const { return (REAL)rsrc[im]; }
+    __device__ REAL protected_store() const { return (REAL)v.ps[im]; }
+    __device__ REAL protected_depth() const { return v.pdep[im]; }
+    __device__ DamRule<REAL> dam_rule() const { return dam_rule_of(v, i); }
+    __device__ REAL dam_inflow() const
+    {
+        return (REAL)v.rti[im] + par<ONE>(v.runoff, CMF_BATCH_RUNOFF, v.batched, i, m, v.M);
+    }
+};
+
 template <typename REAL, bool ONE, bool RES, bool LEV, bool BIF>
 __device__ __forceinline__ void momentum_cell(const Dev<REAL>& v, long i, int m, int kh,
                                               int force_diag)
@@ -282,107 +415,36 @@ __device__ __forceinline__ void momentum_cell(const Dev<REAL>& v, long i, int m,
     const int M = v.M;
     const long im = ix<ONE>(i, m, M);
     const REAL dt = v.dt[m];
-    const REAL gdt = v.g * dt;
     const uint8_t fl = v.flags[i];
-    const bool mouth = fl & CMF_CELL_MOUTH;
-    const bool lev_cell = LEV && (fl & CMF_CELL_LEVEE);
-    const bool res_cell = RES && (fl & CMF_CELL_RESERVOIR);
     const int dn = v.dn[i];
     const long dm = ix<ONE>(dn, m, M);
-
-    const REAL width = par<ONE>(v.rw, CMF_BATCH_RIVER_WIDTH, v.batched, i, m, M);
-    const REAL len = par<ONE>(v.rl, CMF_BATCH_RIVER_LENGTH, v.batched, i, m, M);
-    const REAL bank_h = par<ONE>(v.rh, CMF_BATCH_RIVER_HEIGHT, v.batched, i, m, M);
-    const REAL n_riv = par<ONE>(v.rman, CMF_BATCH_RIVER_MANNING, v.batched, i, m, M);
-    const REAL n_fld = par<ONE>(v.fman, CMF_BATCH_FLOOD_MANNING, v.batched, i, m, M);
-    const REAL elev = v.celv[i];
-    const REAL dx = v.dnd[i];
-    const REAL q_riv_old = v.rout[im];
-    const REAL q_fld_old = v.fout[im];
-    const REAL h_riv = v.rdep[im];
-    const REAL h_fld = v.fdep[im];
-    const REAL hr_before = v.rcsd[im];
-    const REAL hf_before = v.fcsd[im];
-    const REAL af_before = v.fcsa[im];
-    const REAL s_fld = (REAL)fsrc[im];
-
-    // water surfaces: this cell's over its river bed; downstream the next
-    // cell's, or the sea at this catchment's elevation for a mouth
-    const REAL bed = elev - bank_h;
-    const REAL eta = h_riv + bed;
-    const REAL elev_dn = v.celv[dn];
-    const REAL eta_dn = mouth ? elev
-                              : v.rdep[dm] + (elev_dn - par<ONE>(v.rh, CMF_BATCH_RIVER_HEIGHT,
-                                                                 v.batched, dn, m, M));
-    const REAL eta_top = smax(eta, eta_dn);
-    const REAL slope = (eta - eta_dn) / dx;
-
-    // interface state: river flow depth (the own depth at a mouth, whose sea
-    // level sets the slope only), floodplain flow depth and flow area
-    const REAL hr_now = mouth ? h_riv : eta_top - bed;
-    const REAL hf_now = smax((mouth ? eta : eta_top) - elev, REAL(0));
-    const REAL af_now = smax(s_fld / len - h_fld * width, REAL(0));
-    const REAL hr_si = implicit_mean(hr_now, hr_before, REAL(1e-6));
-    const REAL hf_si = implicit_mean(hf_now, hf_before, REAL(1e-6));
-
-    REAL q_riv = REAL(0);
-    if (hr_si > REAL(1e-5) && hr_now * width > REAL(1e-5))
-        q_riv = channel_discharge(q_riv_old, width, n_riv, hr_si, slope, gdt);
-    REAL q_fld = REAL(0);
-    if (hf_si > REAL(1e-5) && af_now > REAL(1e-5)) {
-        const REAL af_si = implicit_mean(af_now, smax(af_before, REAL(1e-6)), REAL(1e-6));
-        q_fld = plain_discharge(q_fld_old, af_si, n_fld, hf_si, capped_slope(slope, REAL(0.005)), gdt);
-    }
-    // the floodplain never flows against the river
-    if (q_riv * q_fld < REAL(0)) q_fld = REAL(0);
-
-    // river storage, read only where a rule below needs it
-    REAL s_riv = REAL(0);
-    bool have_s_riv = false;
-    auto river_store = [&]() -> REAL {
-        if (!have_s_riv) {
-            s_riv = (REAL)rsrc[im];
-            have_s_riv = true;
-        }
-        return s_riv;
-    };
-    // backwater into the cell draws at most 5 % of what it holds per sub-step
-    if (q_riv < REAL(0) && !mouth) {
-        const REAL held = river_store() + s_fld + (lev_cell ? (REAL)v.ps[im] : REAL(0));
-        const REAL rate = smin(REAL(0.05) * held / ((-q_riv - q_fld) * dt), REAL(1));
-        q_riv *= rate;
-        q_fld *= rate;
-    }
-    if (RES && (fl & CMF_CELL_DAM_UPSTREAM)) {
-        const REAL bed_slope = smax((elev - elev_dn) / dx, v.min_kin);
-        kinematic_outflow(bed_slope, len, h_riv, h_fld, river_store(), s_fld, width, n_riv, n_fld,
-                          dt, q_riv, q_fld);
-    }
-    if (res_cell) {
-        // the release replaces the routed flux; the limiter gathers fluxes,
-        // so nothing scattered before needs undoing
-        const int slot = v.rslot[i];
-        const DamRule<REAL> rule{v.rcons[slot], v.radj[slot], v.remerg[slot],
-                                 v.rnout[slot], v.raout[slot], v.rfcout[slot]};
-        const REAL inflow = (REAL)v.rti[im] + par<ONE>(v.runoff, CMF_BATCH_RUNOFF, v.batched, i, m, M);
-        q_riv = dam_release(rule, river_store() + s_fld, inflow, dt);
-        q_fld = REAL(0);
-    }
-
-    v.qu[im] = {q_riv, q_fld};
-    v.rcsd[im] = hr_now;
-    v.fcsd[im] = hf_now;
-    v.fcsa[im] = af_now;
-
-    if (st.diag) {
-        if (v.wse) v.wse[im] = eta;
-        if (v.pwse) v.pwse[im] = lev_cell ? smin(elev + v.pdep[im], eta) : eta;
-        if (v.tsto) {
-            const REAL held = res_cell ? river_store() + s_fld
-                                       : river_store() + s_fld + (lev_cell ? (REAL)v.ps[im] : REAL(0));
-            v.tsto[im] = (double)held;
-        }
-    }
+    MomentumCell<REAL> c;
+    c.width = par<ONE>(v.rw, CMF_BATCH_RIVER_WIDTH, v.batched, i, m, M);
+    c.len = par<ONE>(v.rl, CMF_BATCH_RIVER_LENGTH, v.batched, i, m, M);
+    c.bank_h = par<ONE>(v.rh, CMF_BATCH_RIVER_HEIGHT, v.batched, i, m, M);
+    c.n_riv = par<ONE>(v.rman, CMF_BATCH_RIVER_MANNING, v.batched, i, m, M);
+    c.n_fld = par<ONE>(v.fman, CMF_BATCH_FLOOD_MANNING, v.batched, i, m, M);
+    c.elev = v.celv[i];
+    c.dx = v.dnd[i];
+    c.q_riv = v.rout[im];
+    c.q_fld = v.fout[im];
+    c.h_riv = v.rdep[im];
+    c.h_fld = v.fdep[im];
+    c.hr_before = v.rcsd[im];
+    c.hf_before = v.fcsd[im];
+    c.af_before = v.fcsa[im];
+    c.s_fld = (REAL)fsrc[im];
+    c.elev_dn = v.celv[dn];
+    c.eta_dn = (fl & CMF_CELL_MOUTH)
+                   ? c.elev
+                   : v.rdep[dm] + (c.elev_dn - par<ONE>(v.rh, CMF_BATCH_RIVER_HEIGHT, v.batched, dn, m, M));
+    const GlobalRare<REAL, ONE> rare{v, rsrc, i, im, m};
+    const MomentumRates<REAL> r = momentum_rates<REAL, RES, LEV>(c, fl, dt, v.g, v.min_kin, rare);
+    v.qu[im] = {r.q_riv, r.q_fld};
+    v.rcsd[im] = r.h_riv;
+    v.fcsd[im] = r.h_fld;
+    v.fcsa[im] = r.a_fld;
+    if (st.diag) momentum_diagnostics<REAL, RES, LEV>(v, c.elev, c.s_fld, fl, im, r.eta, rare);
 }
 
 // ---------------------------------------------------------------------------
@@ -487,6 +549,36 @@ __global__ void __launch_bounds__(256, CMF_MOMENTUM_MIN_BLOCKS(REAL, ONE)) k_mom
 // outflow.cu:170-174, reservoir.cu:273-277/320-324, bifurcation.cu:125-128
 // gathered instead of scattered).
 // ---------------------------------------------------------------------------
+// Adds to `og` what a path with summed flux s takes out of its end e (odd: the
+// second end).
+template <typename REAL>
+__device__ __forceinline__ double outgoing_path(double og, REAL s, int e, REAL ts)
+{
+    if (e & 1) og += (double)(-fmin(s, (REAL)0) * ts);
+    else og += (double)(fmax(s, (REAL)0) * ts);
+    return og;
+}
+
+// Adds to `og` what the bifurcation paths of cell x take out of it.
+template <typename REAL, bool ONE>
+__device__ __forceinline__ double outgoing_paths(const Dev<REAL>& v, double og, long x, int m, REAL ts)
+{
+    const int b0 = v.bptr[x], b1 = v.bptr[x + 1];
+    for (int b = b0; b < b1; ++b) {
+        const int e = v.bpaths[b];
+        og = outgoing_path(og, v.bsum[ix<ONE>(e >> 1, m, v.M)], e, ts);
+    }
+    return og;
+}
+
+// Rate at which a cell holding `held` can meet its outgoing volume.
+template <typename REAL>
+__device__ __forceinline__ REAL limit_rate_from(REAL outgoing, double held)
+{
+    const REAL rate_storage = (REAL)held;
+    return (outgoing > (REAL)1e-8) ? fmin(rate_storage / outgoing, (REAL)1.0) : (REAL)1.0;
+}
+
 template <typename REAL, bool ONE, bool BIF>
 __device__ __forceinline__ REAL outgoing_of(const Dev<REAL>& v, long x, int m, REAL ts,
                                             REAL qr, REAL qf)
@@ -515,15 +607,7 @@ __device__ __forceinline__ REAL outgoing_of(const Dev<REAL>& v, long x, int m, R
             }
         }
     }
-    if (BIF && (v.flags[x] & CMF_CELL_BIFURCATION)) {
-        const int b0 = v.bptr[x], b1 = v.bptr[x + 1];
-        for (int b = b0; b < b1; ++b) {
-            const int e = v.bpaths[b];
-            REAL s = v.bsum[ix<ONE>(e >> 1, m, M)];
-            if (e & 1) og += (double)(-fmin(s, (REAL)0) * ts);
-            else og += (double)(fmax(s, (REAL)0) * ts);
-        }
-    }
+    if (BIF && (v.flags[x] & CMF_CELL_BIFURCATION)) og = outgoing_paths<REAL, ONE>(v, og, x, m, ts);
     return (REAL)og;
 }
 
@@ -534,8 +618,7 @@ __device__ __forceinline__ REAL limit_rate_of(const Dev<REAL>& v, const double* 
     const long xm = ix<ONE>(x, m, v.M);
     const pair_t<REAL> q = v.qu[xm];
     REAL outgoing = outgoing_of<REAL, ONE, BIF>(v, x, m, ts, q.x, q.y);
-    REAL rate_storage = (REAL)(rsrc[xm] + fsrc[xm]);
-    return (outgoing > (REAL)1e-8) ? fmin(rate_storage / outgoing, (REAL)1.0) : (REAL)1.0;
+    return limit_rate_from(outgoing, rsrc[xm] + fsrc[xm]);
 }
 
 // ---------------------------------------------------------------------------
@@ -620,6 +703,45 @@ __device__ __forceinline__ void block_budget(double (&val)[kBudgetTerms], double
     }
 }
 
+// Flux q of an upstream cell after the limiter: by its own rate, or by the
+// downstream cell's when it flows backwards.  In fp64 the product is rounded
+// by itself, so that the inflow sums do not depend on whether the compiler
+// fuses it into them (in fp32 the widening to the sums' type keeps it apart).
+template <typename REAL>
+__device__ __forceinline__ REAL limited_flux(REAL q, REAL lr_up, REAL lr_dn)
+{
+    if constexpr (sizeof(REAL) == 8) return __dmul_rn(q, q >= 0.0 ? lr_up : lr_dn);
+    else return q >= (REAL)0.0 ? q * lr_up : q * lr_dn;
+}
+
+// What a path with raw flux `raw` takes from its end e (odd: the second end),
+// whose limit rate is lr_i and whose other end's is lr_o.
+template <typename REAL>
+__device__ __forceinline__ double path_net(REAL raw, int e, REAL lr_i, REAL lr_o)
+{
+    const REAL lr_c = (e & 1) ? lr_o : lr_i;
+    const REAL lr_d = (e & 1) ? lr_i : lr_o;
+    const REAL net = (raw >= (REAL)0) ? raw * lr_c : raw * lr_d;
+    return (e & 1) ? (double)(-net) : (double)net;
+}
+
+// Bifurcation net outflow of cell i, whose limit rate is lr_i
+// (bifurcation.cu:131-156 gathered over the cell's path ends).
+template <typename REAL, bool ONE>
+__device__ __forceinline__ double path_net_of(const Dev<REAL>& v, long i, int m, REAL lr_i)
+{
+    double gb = 0.0;
+    const int b0 = v.bptr[i], b1 = v.bptr[i + 1];
+    for (int b = b0; b < b1; ++b) {
+        const int e = v.bpaths[b];
+        const int p = e >> 1;
+        const REAL raw = v.braw[ix<ONE>(p, m, v.M)];
+        const int other = (e & 1) ? v.bci[p] : v.bdi[p];
+        gb += path_net(raw, e, lr_i, v.lrs[ix<ONE>(other, m, v.M)]);
+    }
+    return gb;
+}
+
 // ---------------------------------------------------------------------------
 // k_stage: cell part
 // ---------------------------------------------------------------------------
@@ -686,8 +808,8 @@ __device__ __forceinline__ void stage_cell(const Dev<REAL>& v, long i, int m, in
 #pragma unroll
         for (int j = 0; j < U; ++j) {
             if (cb + j < c1) {
-                const REAL ur = (cr[j] >= (REAL)0.0) ? cr[j] * cl[j] : cr[j] * lr_i;
-                const REAL uf = (cf[j] >= (REAL)0.0) ? cf[j] * cl[j] : cf[j] * lr_i;
+                const REAL ur = limited_flux(cr[j], cl[j], lr_i);
+                const REAL uf = limited_flux(cf[j], cl[j], lr_i);
                 rin += (double)ur;
                 fin += (double)uf;
                 if (res_cell) rti += (double)(ur + uf);
@@ -702,22 +824,8 @@ __device__ __forceinline__ void stage_cell(const Dev<REAL>& v, long i, int m, in
     const REAL rout = (qr >= (REAL)0.0) ? qr * lr_i : qr * lr_dn;
     const REAL fout = (qf >= (REAL)0.0) ? qf * lr_i : qf * lr_dn;
 
-    // bifurcation net flux of this cell (bifurcation.cu:131-156 gathered)
     double gb = 0.0;
-    if (BIF && (fl & CMF_CELL_BIFURCATION)) {
-        const int b0 = v.bptr[i], b1 = v.bptr[i + 1];
-        for (int b = b0; b < b1; ++b) {
-            const int e = v.bpaths[b];
-            const int p = e >> 1;
-            const REAL raw = v.braw[ix<ONE>(p, m, M)];
-            const int other = (e & 1) ? v.bci[p] : v.bdi[p];
-            const REAL lr_o = v.lrs[ix<ONE>(other, m, M)];
-            const REAL lr_c = (e & 1) ? lr_o : lr_i;
-            const REAL lr_d = (e & 1) ? lr_i : lr_o;
-            const REAL net = (raw >= (REAL)0) ? raw * lr_c : raw * lr_d;
-            gb += (e & 1) ? (double)(-net) : (double)net;
-        }
-    }
+    if (BIF && (fl & CMF_CELL_BIFURCATION)) gb = path_net_of<REAL, ONE>(v, i, m, lr_i);
 
     // continuity and flood stage; levee cells are re-partitioned afterwards
     // by k_levee, which conserves river + flood + protected storage, so the
@@ -830,6 +938,60 @@ __device__ __forceinline__ void advance_step(int* ctl, cudaGraphConditionalHandl
 // levee cells are a scattered minority, and running their long scan inside
 // k_stage would stretch every CTA of the much larger catchment grid.
 // ---------------------------------------------------------------------------
+// Re-partition of a levee cell on its plan-time marks; `flood_depth` supplies
+// the flood depth, which only an overtopped levee reads.
+template <typename REAL, typename Depth, typename FloodDepth>
+__device__ __forceinline__ int levee_by_marks(LeveeState<double, REAL>& lst, const LeveeMarks<REAL, REAL>& mk,
+                                              REAL rw, REAL rh, REAL rl, REAL crown, REAL frac, REAL base,
+                                              int K, Depth depth, FloodDepth flood_depth)
+{
+    // the overtopped test of levee_apply
+    const REAL total = narrow<REAL>(lst.rs + lst.fs);
+    const REAL bank = xmul(xmul(rl, rw), rh);
+    if (total >= bank && total >= mk.s_crown) lst.fdep = flood_depth();
+    return levee_apply<0>(lst, mk, rw, rh, rl, crown, frac, base, K, depth);
+}
+
+// Re-partition of levee li, in cell ci: `lst` holds the cell's river and flood
+// storage, and the regime that applied is returned; `flood_depth` supplies the
+// cell's flood depth where a regime reads it.
+template <typename REAL, bool ONE, typename FloodDepth>
+__device__ __forceinline__ int levee_repartition(const Dev<REAL>& v, long li, long ci, int m,
+                                                 LeveeState<double, REAL>& lst, FloodDepth flood_depth)
+{
+    // static fields from the levee-indexed copies where the plan keeps
+    // them (coalesced over the levee list), else from the cells
+    const REAL* row = v.lpk_tbl ? v.lpk_tbl + li * (long)v.K : v.tbl + ci * (long)v.K;
+    auto depth = [row](int l) { return row[l]; };
+    REAL rh, rw, rl;
+    if (v.lpk_geo) {
+        rh = v.lpk_geo[li];
+        rw = v.lpk_geo[v.NLV + li];
+        rl = v.lpk_geo[2 * v.NLV + li];
+    } else {
+        rh = par<ONE>(v.rh, CMF_BATCH_RIVER_HEIGHT, v.batched, ci, m, v.M);
+        rw = par<ONE>(v.rw, CMF_BATCH_RIVER_WIDTH, v.batched, ci, m, v.M);
+        rl = par<ONE>(v.rl, CMF_BATCH_RIVER_LENGTH, v.batched, ci, m, v.M);
+    }
+    const REAL crown = v.lcrown[li], frac = v.lfrac[li], base = v.lbase[li];
+    if (v.lmk) {
+        // the plan's marks: the row is read only while the protected
+        // side fills
+        const long n = v.NLV;
+        LeveeMarks<REAL, REAL> mk;
+        mk.s_base = v.lmk[li];
+        mk.s_crown = v.lmk[n + li];
+        mk.s_top = v.lmk[2 * n + li];
+        mk.s_first = v.lmk[3 * n + li];
+        mk.dw = v.lmk[4 * n + li];
+        mk.dist = v.lmk[5 * n + li];
+        return levee_by_marks<REAL>(lst, mk, rw, rh, rl, crown, frac, base, v.K, depth, flood_depth);
+    } else {
+        lst.fdep = flood_depth();
+        return levee_partition<0>(lst, rw, rh, rl, v.ca[ci], crown, frac, base, v.K, depth);
+    }
+}
+
 // One levee (list index li) of member m: re-partition of its cell's
 // flood-stage result, as k_levee and the persistent interval kernel run it.
 template <typename REAL, bool ONE>
@@ -852,42 +1014,7 @@ __device__ __forceinline__ void levee_cell(const Dev<REAL>& v, long li, int m, i
     lst.rdep = REAL(0);
     lst.fdep = REAL(0);
     lst.ffr = REAL(0);
-    // static fields from the levee-indexed copies where the plan keeps
-    // them (coalesced over the levee list), else from the cells
-    const REAL* row = v.lpk_tbl ? v.lpk_tbl + li * (long)v.K : v.tbl + ci * (long)v.K;
-    auto depth = [row](int l) { return row[l]; };
-    REAL rh, rw, rl;
-    if (v.lpk_geo) {
-        rh = v.lpk_geo[li];
-        rw = v.lpk_geo[v.NLV + li];
-        rl = v.lpk_geo[2 * v.NLV + li];
-    } else {
-        rh = par<ONE>(v.rh, CMF_BATCH_RIVER_HEIGHT, v.batched, ci, m, v.M);
-        rw = par<ONE>(v.rw, CMF_BATCH_RIVER_WIDTH, v.batched, ci, m, v.M);
-        rl = par<ONE>(v.rl, CMF_BATCH_RIVER_LENGTH, v.batched, ci, m, v.M);
-    }
-    const REAL crown = v.lcrown[li], frac = v.lfrac[li], base = v.lbase[li];
-    int regime;
-    if (v.lmk) {
-        // the plan's marks: the row is read only while the protected
-        // side fills
-        const long n = v.NLV;
-        LeveeMarks<REAL, REAL> mk;
-        mk.s_base = v.lmk[li];
-        mk.s_crown = v.lmk[n + li];
-        mk.s_top = v.lmk[2 * n + li];
-        mk.s_first = v.lmk[3 * n + li];
-        mk.dw = v.lmk[4 * n + li];
-        mk.dist = v.lmk[5 * n + li];
-        // the overtopped test of levee_apply, to fetch the flood depth it reads
-        const REAL total = narrow<REAL>(lst.rs + lst.fs);
-        const REAL bank = xmul(xmul(rl, rw), rh);
-        if (total >= bank && total >= mk.s_crown) lst.fdep = v.fdep[cm];
-        regime = levee_apply<0>(lst, mk, rw, rh, rl, crown, frac, base, v.K, depth);
-    } else {
-        lst.fdep = v.fdep[cm];
-        regime = levee_partition<0>(lst, rw, rh, rl, v.ca[ci], crown, frac, base, v.K, depth);
-    }
+    const int regime = levee_repartition<REAL, ONE>(v, li, ci, m, lst, [&]() { return v.fdep[cm]; });
     v.ps[cm] = lst.ps;
     v.pdep[cm] = lst.pdep;
     if (regime == kLeveeOvertopped) {
@@ -1057,6 +1184,16 @@ __global__ void k_barrier_timeout_probe(int* ctl, int* status, unsigned long lon
 // ---------------------------------------------------------------------------
 // CFL sub-step count (adaptive_time.cu:19-48), per member.
 // ---------------------------------------------------------------------------
+template <typename REAL>
+__device__ __forceinline__ int cfl_steps(REAL dist, REAL raw_depth, REAL alpha, REAL g, REAL max_dt, REAL outer_dt)
+{
+    REAL depth = fmax(raw_depth, (REAL)0.01);
+    REAL dt = alpha * dist / sqrt(g * depth);
+    if (max_dt > (REAL)0) dt = fmin(dt, max_dt);
+    REAL dt_clamped = fmin(dt, outer_dt);
+    return (int)(floor(outer_dt / dt_clamped - (REAL)0.01) + (REAL)1.0);
+}
+
 template <typename REAL, bool ONE, bool RES>
 __global__ void __launch_bounds__(256) k_cfl(const Dev<REAL> v)
 {
@@ -1067,14 +1204,7 @@ __global__ void __launch_bounds__(256) k_cfl(const Dev<REAL> v)
         long i = split_member<ONE>(v, t, m);
         bool skip = RES && (v.flags[i] & CMF_CELL_DAM_RELATED);
         if (!skip) {
-            REAL dist = v.dnd[i];
-            REAL raw_depth = v.rdep[ix<ONE>(i, m, v.M)];
-            REAL depth = fmax(raw_depth, (REAL)0.01);
-            REAL dt = v.cfl_alpha * dist / sqrt(v.g * depth);
-            if (v.max_dt > (REAL)0) dt = fmin(dt, v.max_dt);
-            REAL outer_dt = v.outer[0];
-            REAL dt_clamped = fmin(dt, outer_dt);
-            n_steps = (int)(floor(outer_dt / dt_clamped - (REAL)0.01) + (REAL)1.0);
+            n_steps = cfl_steps(v.dnd[i], v.rdep[ix<ONE>(i, m, v.M)], v.cfl_alpha, v.g, v.max_dt, v.outer[0]);
         }
     }
     if (ONE) {
@@ -1114,7 +1244,13 @@ __global__ void k_interval_begin(const Dev<REAL> v, double outer_seconds, int ad
         v.outer[0] = (REAL)outer_seconds;
         v.ctl[kCtlStep] = 0;
         v.ctl[kCtlBlocksDone] = 0;
+        if (v.rflag) {
+            v.ctl[kCtlCflMax] = 0;
+            v.ctl[kCtlAbort] = 0;
+        }
     }
+    if (v.rflag)
+        for (int q = m; q < kResidentMaxTiles; q += blockDim.x) v.rflag[q] = 0;
     for (int q = m; q < v.M; q += blockDim.x)
         if (adaptive) v.nsub[q] = 0;
 }
@@ -1268,6 +1404,15 @@ __device__ __forceinline__ double stat_value(const Dev<REAL>& v, int var, long t
     }
 }
 
+// Folds value x of a sub-step of length dt into the accumulator of statistic op.
+__device__ __forceinline__ void fold_stat(double* o, int op, double x, double dt)
+{
+    const double acc = *o;
+    if (op == CMF_STAT_MEAN) *o = __dadd_rn(acc, __dmul_rn(x, dt));
+    else if (op == CMF_STAT_MAX) *o = (x > acc || x != x) ? x : acc;
+    else *o = (x < acc || x != x) ? x : acc;
+}
+
 // kh >= 0: host step index; kh == -1: the step that the last kernel of the
 // sub-step just finished (the device counter was advanced by it).
 template <typename REAL, bool ONE>
@@ -1285,12 +1430,7 @@ __global__ void __launch_bounds__(256) k_stats_accumulate(const Dev<REAL> v, con
     for (int q = 0; q < a.count; ++q) {
         const int op = a.op[q];
         if (op == CMF_STAT_LAST) continue;
-        const double x = stat_value(v, a.var[q], t, i, k);
-        double* o = a.out[q] + t;
-        const double acc = *o;
-        if (op == CMF_STAT_MEAN) *o = __dadd_rn(acc, __dmul_rn(x, dt));
-        else if (op == CMF_STAT_MAX) *o = (x > acc || x != x) ? x : acc;
-        else *o = (x < acc || x != x) ? x : acc;
+        fold_stat(a.out[q] + t, op, stat_value(v, a.var[q], t, i, k), dt);
     }
 }
 

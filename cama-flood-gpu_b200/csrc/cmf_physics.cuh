@@ -129,40 +129,56 @@ struct PathEnds {
     T store_a, store_b;  // total storage of the end cells
 };
 
-// Unlimited per-level fluxes of one path.  Level l carries water above its
-// sill elevation; with levees, level 0 sees the river surfaces and the higher
-// levels the protected-side surfaces, and the semi-implicit depth falls back
-// to the new depth where the geometric mean vanishes; without levees the
-// previous depth is floored at 0.01 m.  `lv` supplies the level's sill
-// elevation, width, Manning coefficient, previous flux and previous depth,
-// loaded only when used, and receives each level's new depth
-// (lv.new_depth).  Writes the unlimited fluxes; returns their sum.
+// Unlimited flux of one level of a path, and its new depth h.  Level l carries
+// water above its sill elevation; with levees, level 0 sees the river surfaces
+// and the higher levels the protected-side surfaces, and the semi-implicit
+// depth falls back to the new depth where the geometric mean vanishes; without
+// levees the previous depth is floored at 0.01 m.  `top` and `ptop` are the
+// higher of the two ends' surfaces, `lv` supplies the level's sill elevation,
+// width, Manning coefficient, previous flux and previous depth, loaded only
+// when used.
+template <bool LEVEE, typename T, typename P, typename Levels>
+__device__ __forceinline__ T path_level_flux(const Levels& lv, int l, T top, T ptop, T slope, P gdt, T& h)
+{
+    const T surface = (LEVEE && l > 0) ? ptop : top;
+    h = smax(surface - lv.sill(l), T(0));
+    T h_si;
+    if (LEVEE) {
+        h_si = h;
+        if (l == 0) {
+            h_si = ssqrt(h * lv.depth(0));
+            if (val(h_si) <= P(0)) h_si = h;
+        }
+    } else {
+        h_si = smax(ssqrt(h * lv.depth(l)), ssqrt(h * P(0.01)));
+    }
+    if (!(val(h_si) > P(1e-5))) return T(0);
+    return channel_discharge(lv.flux(l), lv.width(l), lv.manning(l), h_si, slope, gdt);
+}
+
+// The path's surface slope, limited.
+template <typename T, typename P>
+__device__ __forceinline__ T path_slope(const PathEnds<T>& e, P length)
+{
+    return capped_slope((e.eta_a - e.eta_b) / length, P(0.005));
+}
+
+// Unlimited fluxes of every level of a path; `lv` receives each level's new
+// depth (lv.new_depth).  Returns their sum.
 template <bool LEVEE, int LMAX, typename T, typename P, typename Levels>
 __device__ __forceinline__ T path_level_fluxes(const Levels& lv, int L, const PathEnds<T>& e,
                                                P length, P gdt, T (&flux)[LMAX])
 {
     const T top = smax(e.eta_a, e.eta_b);
     const T ptop = LEVEE ? smax(e.peta_a, e.peta_b) : top;
-    const T slope = capped_slope((e.eta_a - e.eta_b) / length, P(0.005));
+    const T slope = path_slope(e, length);
     T sum = T(0);
 #pragma unroll
     for (int l = 0; l < LMAX; ++l) {
         T q = T(0);
         if (l < L) {
-            const T surface = (LEVEE && l > 0) ? ptop : top;
-            const T h = smax(surface - lv.sill(l), T(0));
-            T h_si;
-            if (LEVEE) {
-                h_si = h;
-                if (l == 0) {
-                    h_si = ssqrt(h * lv.depth(0));
-                    if (val(h_si) <= P(0)) h_si = h;
-                }
-            } else {
-                h_si = smax(ssqrt(h * lv.depth(l)), ssqrt(h * P(0.01)));
-            }
-            if (val(h_si) > P(1e-5))
-                q = channel_discharge(lv.flux(l), lv.width(l), lv.manning(l), h_si, slope, gdt);
+            T h;
+            q = path_level_flux<LEVEE>(lv, l, top, ptop, slope, gdt, h);
             sum = sum + q;
             lv.new_depth(l, h);
         }

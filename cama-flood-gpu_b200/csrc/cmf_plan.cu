@@ -17,6 +17,7 @@
 
 #include "cmfb200.h"
 #include "cmf_device.cuh"
+#include "cmf_resident.cuh"
 
 #include <cstdint>
 #include <cstring>
@@ -29,6 +30,11 @@ using namespace cmf;
 namespace {
 
 constexpr int kDefaultBlock = 256;
+// Fewest cells per tile of the resident kernel: with fewer, more neighbours lie
+// in other tiles; with more, a small network leaves SMs idle (4,000 full-physics
+// catchments: 14.0, 13.3, 12.1, 14.1 and 14.5 us per sub-step at 32, 64, 128,
+// 256 and 512 cells).
+constexpr int kResidentMinTile = 128;
 
 struct KernelSet {
     const void* momentum;
@@ -44,6 +50,7 @@ struct KernelSet {
     const void* stats_reset;
     const void* stats_fin;
     const void* persist;  // persistent interval kernel (one member, no budget), else null
+    const void* resident; // resident interval kernel (one member, no budget), else null
 };
 
 template <typename REAL, bool ONE, bool RES, bool LEV, bool BIF, bool BUD>
@@ -62,8 +69,12 @@ KernelSet make_set()
     k.stats_acc = (const void*)k_stats_accumulate<REAL, ONE>;
     k.stats_reset = (const void*)k_stats_reset<REAL, ONE>;
     k.stats_fin = (const void*)k_stats_finalize<REAL, ONE>;
-    if constexpr (ONE && !BUD) k.persist = (const void*)k_persistent<REAL, RES, LEV, BIF>;
-    else k.persist = nullptr;
+    if constexpr (ONE && !BUD) {
+        k.persist = (const void*)k_persistent<REAL, RES, LEV, BIF>;
+        k.resident = (const void*)k_resident<REAL, RES, LEV, BIF>;
+    } else {
+        k.persist = k.resident = nullptr;
+    }
     return k;
 }
 
@@ -100,8 +111,21 @@ struct Layout {
     size_t base_total;  // the regions every caller needs
     // levee-indexed copies that plans keep (after base_total; none without levees)
     size_t lpk_tbl, lpk_geo, lmk;
+    // resident kernel: flags and exchanged words (none where it cannot run)
+    size_t rflag, xflux, xeta, xrate, xend, xsum, xprate, x_end;
     size_t total;
 };
+
+// Whether a view's network can fit the SMs' shared memory at all: one member,
+// no budget, and at most kResidentMaxTiles tiles of 228 KB.  plan_resident
+// decides with the device's own figures.
+bool may_be_resident(const CmfView* v)
+{
+    const size_t real = (v->features & CMF_FEAT_FP64) ? 8 : 4;
+    const size_t cell = 2 * 8 + kResidentFields * real + 4 * sizeof(int) + 1;
+    return v->num_members == 1 && !(v->features & CMF_FEAT_BUDGET) &&
+           (size_t)v->num_catchments * cell <= (size_t)kResidentMaxTiles * 228 * 1024;
+}
 
 Layout layout_of(const CmfView* v, int cell_blocks)
 {
@@ -124,6 +148,18 @@ Layout layout_of(const CmfView* v, int cell_blocks)
     L.lpk_tbl = o; o = align_up(o + nlv * (size_t)v->num_flood_levels * real);
     L.lpk_geo = o; o = align_up(o + 3 * nlv * real);
     L.lmk = o; o = align_up(o + 6 * nlv * real);
+    const bool resident = may_be_resident(v);
+    const size_t word = real / 4 * 8;  // a value with its epochs
+    const size_t nw = resident ? (size_t)v->num_catchments * word : 0;
+    const size_t pw = resident && (v->features & CMF_FEAT_BIFURCATION) ? (size_t)v->num_bifurcation_paths * word : 0;
+    L.rflag = o; o = align_up(o + kResidentMaxTiles * sizeof(unsigned));
+    L.xflux = o; o = align_up(o + 2 * nw);
+    L.xeta = o; o = align_up(o + nw);
+    L.xrate = o; o = align_up(o + nw);
+    L.xend = o; o = align_up(o + 3 * pw);
+    L.xsum = o; o = align_up(o + 2 * pw);
+    L.xprate = o; o = align_up(o + 2 * pw);
+    L.x_end = o;
     L.total = o;
     return L;
 }
@@ -168,6 +204,10 @@ struct CmfPlan {
     // persistent interval kernel instead of the interval graph
     bool persistent;
     int persist_grid;
+    // resident interval kernel: its tiles (0: the network does not fit)
+    ResidentArgs resident;
+    int resident_tiles;
+    int resident_threads;
 };
 
 namespace {
@@ -270,6 +310,15 @@ void fill_dev(CmfPlan* p, const Layout& L, bool packed)
     d.status = v.status;
     d.qu = (pair_t<REAL>*)(ws + L.qu);
     d.lrs = (REAL*)(ws + L.lrs);
+    if (packed && may_be_resident(&v)) {
+        d.rflag = (unsigned*)(ws + L.rflag);
+        d.xflux = (unsigned long long*)(ws + L.xflux);
+        d.xeta = (unsigned long long*)(ws + L.xeta);
+        d.xrate = (unsigned long long*)(ws + L.xrate);
+        d.xend = (unsigned long long*)(ws + L.xend);
+        d.xsum = (unsigned long long*)(ws + L.xsum);
+        d.xprate = (unsigned long long*)(ws + L.xprate);
+    }
     if (packed && d.NLV > 0) {
         d.lpk_tbl = (REAL*)(ws + L.lpk_tbl);
         const int geo = CMF_BATCH_RIVER_HEIGHT | CMF_BATCH_RIVER_WIDTH | CMF_BATCH_RIVER_LENGTH;
@@ -537,6 +586,80 @@ int interval_direct(CmfPlan* p, cudaStream_t s, double T, int fixed_n)
     return CMF_OK;
 }
 
+// Tiles of the resident kernel for this plan's network, if it fits: one tile
+// per SM, as many cells as spread the network over the SMs, and the
+// floodplain rows in shared memory too where they find room.  It is taken
+// wherever it fits, because it was the faster form at every such size: a daily
+// interval through the interval graph and through this kernel, us per
+// sub-step: 60k plain 27.2 / 7.0, 250k full physics 45.7 / 21.2, 100k full
+// physics with two statistics 40.3 / 13.8, 30k full physics fp64 37.4 / 16.7;
+// an hour of 4k full physics 32.1 / 11.2.
+int plan_resident(CmfPlan* p, const Layout& L)
+{
+    p->resident_tiles = 0;
+    const CmfView& v = p->view;
+    const int geo = CMF_BATCH_RIVER_HEIGHT | CMF_BATCH_RIVER_WIDTH | CMF_BATCH_RIVER_LENGTH;
+    if (!p->ks.resident || !may_be_resident(&v) || (p->levee_blocks > 0 && (v.batched_mask & geo))) return CMF_OK;
+    int dev = 0, coop = 0, sms = 0, smem = 0, rc;
+    if ((rc = check_cuda(cudaGetDevice(&dev))) != CMF_OK) return rc;
+    if ((rc = check_cuda(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev))) != CMF_OK) return rc;
+    if ((rc = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev))) != CMF_OK) return rc;
+    if ((rc = check_cuda(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev))) != CMF_OK)
+        return rc;
+    cudaFuncAttributes fa;
+    if ((rc = check_cuda(cudaFuncGetAttributes(&fa, p->ks.resident))) != CMF_OK) return rc;
+    const int room = smem - (int)fa.sharedSizeBytes;
+    const int max_tiles = sms < kResidentMaxTiles ? sms : kResidentMaxTiles;
+    const long spread = ceil_div((long)v.num_catchments, max_tiles);
+    if (!coop) return CMF_OK;
+    int tile = spread > kResidentMinTile ? (int)spread : kResidentMinTile;
+    tile = (tile + 31) / 32 * 32;
+    const int tiles = ceil_div((long)v.num_catchments, tile);
+    ResidentArgs& a = p->resident;
+    std::memset(&a, 0, sizeof(a));
+    a.tile = tile;
+    char* ws = (char*)v.workspace;
+    void* args[] = {p->dev, &tile};
+    const void* scan = p->fp64 ? (const void*)k_resident_scan<double> : (const void*)k_resident_scan<float>;
+    if ((rc = launch(scan, tiles, 256, args, 0)) != CMF_OK) return rc;
+    if ((rc = check_cuda(cudaMemcpy(&a.most, (int*)(ws + L.ctl) + kCtlTileMax, sizeof(a.most),
+                                    cudaMemcpyDeviceToHost))) != CMF_OK)
+        return rc;
+    const int real = p->fp64 ? 8 : 4;
+    resident_layout(a, real, v.num_flood_levels, v.num_bifurcation_levels, true);
+    if (a.bytes > room) resident_layout(a, real, v.num_flood_levels, v.num_bifurcation_levels, false);
+    if (a.bytes > room) return CMF_OK;
+    // the attribute is the function's, shared by all plans: always the maximum
+    if ((rc = check_cuda(cudaFuncSetAttribute(p->ks.resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              room))) != CMF_OK)
+        return rc;
+    // a warp per chunk of cells and of paths, as far as they go
+    const int most = p->fp64 ? resident_threads<double>() : resident_threads<float>();
+    const int threads = tile + 32 * ceil_div(a.most.paths, 32 / kPathLanes);
+    p->resident_threads = threads < most ? threads : most;
+    // no word may carry an epoch that this plan will use
+    if ((rc = check_cuda(cudaMemset(ws + L.rflag, 0, L.x_end - L.rflag))) != CMF_OK) return rc;
+    p->resident_tiles = tiles;
+    return CMF_OK;
+}
+
+// One interval through the resident kernel: the prologue, then the whole
+// interval in one cooperative launch.
+int interval_resident(CmfPlan* p, cudaStream_t s, double T, int fixed_n)
+{
+    int rc;
+    {
+        int a = fixed_n <= 0 ? 1 : 0;
+        void* args[] = {p->dev, &T, &a};
+        if ((rc = launch(p->ks.begin, 1, 32, args, s)) != CMF_OK) return rc;
+    }
+    ResidentArgs ra = p->resident;
+    ra.fixed_n = fixed_n;
+    void* args[] = {p->dev, &p->stats, &ra};
+    return check_cuda(cudaLaunchCooperativeKernel(p->ks.resident, dim3(p->resident_tiles),
+                                                   dim3(p->resident_threads), args, p->resident.bytes, s));
+}
+
 // One interval through the persistent kernel: the prologue kernels, then
 // every sub-step in one cooperative launch, then the epilogue.
 int interval_persistent(CmfPlan* p, cudaStream_t s, double T, int fixed_n)
@@ -694,6 +817,10 @@ int cmf_plan_create(const CmfView* view, CmfPlan** out)
             return rc;
         }
     }
+    if ((rc = plan_resident(p, L)) != CMF_OK) {
+        delete p;
+        return rc;
+    }
     *out = p;
     return CMF_OK;
 }
@@ -715,6 +842,12 @@ int cmf_step_interval(CmfPlan* p, void* stream, double outer_seconds, int32_t fi
     if (p->persistent) return interval_persistent(p, s, outer_seconds, fixed);
     if (!p->graph_enabled) return interval_direct(p, s, outer_seconds, fixed);
     int rc;
+    if (p->resident_tiles > 0) {
+        // a stream capture takes the interval graph, as it always has
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone)
+            return interval_resident(p, s, outer_seconds, fixed);
+    }
     const bool adaptive_now = fixed == 0;
     if (p->graph_ready) {
         const bool was_adaptive = p->graph_fixed == 0;
