@@ -60,9 +60,10 @@ template <typename REAL, bool ONE>
 __host__ __device__ constexpr bool stage_row_in_regs() { return !(sizeof(REAL) == 4 && ONE); }
 // k_momentum: 8 CTAs (32 registers) for one fp32 member, where the few bytes
 // it spills cost less than the occupancy they buy (182 -> 161 us per 6M
-// sub-step); fp64 and member-batched variants would spill hundreds of bytes
+// sub-step); 3 (80 registers, no spills) for fp32 members, whose full-physics
+// form would take 86; fp64 would spill hundreds of bytes
 #ifndef CMF_MOMENTUM_MIN_BLOCKS
-#define CMF_MOMENTUM_MIN_BLOCKS(REAL, ONE) ((sizeof(REAL) == 4 && (ONE)) ? 8 : 1)
+#define CMF_MOMENTUM_MIN_BLOCKS(REAL, ONE) (sizeof(REAL) == 4 ? ((ONE) ? 8 : 3) : 1)
 #endif
 
 namespace cmf {
@@ -82,9 +83,12 @@ __host__ __device__ constexpr int child_unroll() { return ONE ? kChildUnroll : C
 constexpr int kMaxBlock = 256;       // threads per CTA (kernels use __launch_bounds__(256))
 constexpr int kBudgetTerms = CMF_BUDGET_TERMS;
 // control words (Dev::ctl)
-constexpr int kCtlStep = 0;       // current sub-step index k
+// The sub-step index has two words, so that no kernel reads the one it sets:
+// k_momentum reads the first and copies it to the second, which the later
+// kernels read, and k_limit sets the first to the second plus one.
+constexpr int kCtlStep = 0;    // index k that k_momentum reads
+constexpr int kCtlStepOf = 2;  // index k that the other kernels of the sub-step read
 constexpr int kCtlMaxSteps = 1;   // max over members of the sub-step count
-constexpr int kCtlBlocksDone = 2; // last-block-done counter of k_stage
 constexpr int kCtlBarrier = 4;    // [4..5]: arrival counter (u64) of the persistent kernel's grid barrier
 constexpr int kCtlAbort = 6;      // set when a grid barrier gave up: every block leaves the interval
 constexpr int kCtlCflMax = 8;     // resident kernel: CFL sub-step count, maximum over the tiles
@@ -227,23 +231,20 @@ __device__ __forceinline__ int upstream_end(const Dev<REAL>& v, long x)
 }
 
 // Member-active test and the per-member last-sub-step flag.
-//   kh >= 0: a host-chosen step index (per-phase entry points);
-//   kh == -1: read the interval's step counter from the device;
+//   kh >= 0: a step index chosen by the caller;
+//   kh == -1: the interval's step counter, word `word` of the control words (one
+//             member only: see tile_step);
 //   kh == -2: every member active, diag only when force_diag == 1.
 // force_diag: 0 = last sub-step of the member, 1 = always, 2 = never.
+template <bool ONE>
 __device__ __forceinline__ bool member_step(const int* ctl, const int* nsub, int kh, int m,
-                                            int force_diag, bool& diag)
+                                            int force_diag, bool& diag, int word)
 {
     if (kh == -2) { diag = force_diag == 1; return true; }
-    int k = kh >= 0 ? kh : ctl[kCtlStep];
+    const int k = ONE && kh == -1 ? ctl[word] : kh;
     int nm = nsub[m];
     diag = (force_diag == 1) || (force_diag == 0 && k == nm - 1);
     return k < nm;
-}
-
-__device__ __forceinline__ int step_index(const int* ctl, int kh)
-{
-    return kh >= 0 ? kh : (kh == -1 ? ctl[kCtlStep] : 0);
 }
 
 // Step index, activity and last-sub-step flag of member m (see member_step).
@@ -257,7 +258,7 @@ struct StepInfo {
 
 template <bool ONE>
 __device__ __forceinline__ StepInfo step_info(const int* ctl, const int* nsub, int kh, int m,
-                                              int force_diag)
+                                              int force_diag, int word)
 {
     StepInfo s;
     if (kh == -2) {
@@ -266,11 +267,21 @@ __device__ __forceinline__ StepInfo step_info(const int* ctl, const int* nsub, i
         s.diag = force_diag == 1;
         return s;
     }
-    s.k = kh >= 0 ? kh : ctl[kCtlStep];
+    s.k = ONE && kh == -1 ? ctl[word] : kh;
     const int nm = nsub[m];
     s.diag = (force_diag == 1) || (force_diag == 0 && s.k == nm - 1);
     s.active = ONE || s.k < nm;
     return s;
+}
+
+// With members, the counter is read once per thread instead of once per member
+// of its tile (64 members x 60k: k_momentum 86 -> 74 us, k_limit 66 -> 62); a
+// single member's thread has one element, and holding the index from the start
+// would only cost it registers.
+template <bool ONE>
+__device__ __forceinline__ int tile_step(const int* ctl, int kh, int word)
+{
+    return !ONE && kh == -1 ? ctl[word] : kh;
 }
 
 // ---------------------------------------------------------------------------
@@ -408,7 +419,7 @@ template <typename REAL, bool ONE, bool RES, bool LEV, bool BIF>
 __device__ __forceinline__ void momentum_cell(const Dev<REAL>& v, long i, int m, int kh,
                                               int force_diag)
 {
-    const StepInfo st = step_info<ONE>(v.ctl, v.nsub, kh, m, force_diag);
+    const StepInfo st = step_info<ONE>(v.ctl, v.nsub, kh, m, force_diag, kCtlStep);
     if (!st.active) return;
     const double* __restrict__ rsrc = (st.k & 1) ? v.rs1 : v.rs0;
     const double* __restrict__ fsrc = (st.k & 1) ? v.fs1 : v.fs0;
@@ -491,7 +502,7 @@ struct PathLevelFields {
 template <typename REAL, bool ONE, bool RES, bool LEV>
 __device__ __forceinline__ void momentum_path(const Dev<REAL>& v, long p, int m, int kh)
 {
-    const StepInfo st = step_info<ONE>(v.ctl, v.nsub, kh, m, 2);
+    const StepInfo st = step_info<ONE>(v.ctl, v.nsub, kh, m, 2, kCtlStep);
     if (!st.active) return;
     const double* rsrc = (st.k & 1) ? v.rs1 : v.rs0;
     const double* fsrc = (st.k & 1) ? v.fs1 : v.fs0;
@@ -522,6 +533,11 @@ __device__ __forceinline__ void momentum_path(const Dev<REAL>& v, long p, int m,
 template <typename REAL, bool ONE, bool RES, bool LEV, bool BIF>
 __global__ void __launch_bounds__(256, CMF_MOMENTUM_MIN_BLOCKS(REAL, ONE)) k_momentum(const Dev<REAL> v, int kh, int force_diag)
 {
+    if (kh == -1) {
+        const int k = v.ctl[kCtlStep];
+        if (blockIdx.x == 0 && threadIdx.x == 0) v.ctl[kCtlStepOf] = k;
+        if (!ONE) kh = k;  // as tile_step
+    }
     const int W = mtile_of<REAL, ONE>(v);
     if (BIF && (int)blockIdx.x >= v.cell_blocks) {
         const long t0 = (long)(blockIdx.x - v.cell_blocks) * blockDim.x + threadIdx.x;
@@ -612,13 +628,14 @@ __device__ __forceinline__ REAL outgoing_of(const Dev<REAL>& v, long x, int m, R
 }
 
 template <typename REAL, bool ONE, bool BIF>
-__device__ __forceinline__ REAL limit_rate_of(const Dev<REAL>& v, const double* rsrc,
-                                              const double* fsrc, long x, int m, REAL ts)
+__device__ __forceinline__ REAL limit_rate_of(const Dev<REAL>& v, const double* __restrict__ rsrc,
+                                              const double* __restrict__ fsrc, long x, int m, REAL ts)
 {
     const long xm = ix<ONE>(x, m, v.M);
     const pair_t<REAL> q = v.qu[xm];
-    REAL outgoing = outgoing_of<REAL, ONE, BIF>(v, x, m, ts, q.x, q.y);
-    return limit_rate_from(outgoing, rsrc[xm] + fsrc[xm]);
+    const double held = rsrc[xm] + fsrc[xm];  // on its way during the gather
+    const REAL outgoing = outgoing_of<REAL, ONE, BIF>(v, x, m, ts, q.x, q.y);
+    return limit_rate_from(outgoing, held);
 }
 
 // ---------------------------------------------------------------------------
@@ -753,13 +770,12 @@ __device__ __forceinline__ void stage_cell(const Dev<REAL>& v, long i, int m, in
     // load's value: the activity test of a single member is static (the
     // interval loop only runs k < n), and the upstream gather is unrolled into
     // independent predicated loads.
-    const StepInfo st = step_info<ONE>(v.ctl, v.nsub, kh, m, force_diag);
+    const StepInfo st = step_info<ONE>(v.ctl, v.nsub, kh, m, force_diag, kCtlStepOf);
     if (!st.active) return;
-    const int k = st.k;
-    const double* __restrict__ rsrc = (k & 1) ? v.rs1 : v.rs0;
-    const double* __restrict__ fsrc = (k & 1) ? v.fs1 : v.fs0;
-    double* __restrict__ rdst = (k & 1) ? v.rs0 : v.rs1;
-    double* __restrict__ fdst = (k & 1) ? v.fs0 : v.fs1;
+    const double* __restrict__ rsrc = (st.k & 1) ? v.rs1 : v.rs0;
+    const double* __restrict__ fsrc = (st.k & 1) ? v.fs1 : v.fs0;
+    double* __restrict__ rdst = (st.k & 1) ? v.rs0 : v.rs1;
+    double* __restrict__ fdst = (st.k & 1) ? v.fs0 : v.fs1;
     const int M = v.M;
     const long im = ix<ONE>(i, m, M);
     const REAL ts = v.dt[m];
@@ -871,7 +887,7 @@ template <typename REAL, bool ONE, bool BIF>
 __device__ __forceinline__ void stage_path(const Dev<REAL>& v, long p, int m, int kh)
 {
     bool diag;
-    if (!member_step(v.ctl, v.nsub, kh, m, 2, diag)) return;
+    if (!member_step<ONE>(v.ctl, v.nsub, kh, m, 2, diag, kCtlStepOf)) return;
     const int ci = v.bci[p], di = v.bdi[p];
     const REAL lr_c = v.lrs[ix<ONE>(ci, m, v.M)];
     const REAL lr_d = v.lrs[ix<ONE>(di, m, v.M)];
@@ -891,17 +907,32 @@ __device__ __forceinline__ void stage_path(const Dev<REAL>& v, long p, int m, in
 template <typename REAL, bool ONE, bool BIF>
 __device__ __forceinline__ void limit_cell(const Dev<REAL>& v, long i, int m, int kh)
 {
-    const StepInfo st = step_info<ONE>(v.ctl, v.nsub, kh, m, 2);
+    const StepInfo st = step_info<ONE>(v.ctl, v.nsub, kh, m, 2, kCtlStepOf);
     if (!st.active) return;
-    const int k = st.k;
-    const double* rsrc = (k & 1) ? v.rs1 : v.rs0;
-    const double* fsrc = (k & 1) ? v.fs1 : v.fs0;
+    const double* rsrc = (st.k & 1) ? v.rs1 : v.rs0;
+    const double* fsrc = (st.k & 1) ? v.fs1 : v.fs0;
     v.lrs[ix<ONE>(i, m, v.M)] = limit_rate_of<REAL, ONE, BIF>(v, rsrc, fsrc, i, m, v.dt[m]);
 }
 
-template <typename REAL, bool ONE, bool BIF>
-__global__ void __launch_bounds__(256, (sizeof(REAL) == 4 ? 8 : 4)) k_limit(const Dev<REAL> v, int kh)
+// Interval loop control inside the interval graph, by the first thread of
+// k_limit: the next sub-step's index, which no kernel of this one reads any
+// more, and the while-condition.  (Counting finished blocks for it in the last
+// kernel cost every block a barrier, a fence and an atomic at its end: 7.72
+// against 6.51 ms for an hour of 2M catchments.  k_stage, which has no register
+// to spare, spilled with it.)
+__device__ __forceinline__ void advance_step(int* ctl, cudaGraphConditionalHandle h)
 {
+    const int next = ctl[kCtlStepOf] + 1;
+    ctl[kCtlStep] = next;
+    cudaGraphSetConditional(h, next < ctl[kCtlMaxSteps] ? 1u : 0u);
+}
+
+template <typename REAL, bool ONE, bool BIF>
+__global__ void __launch_bounds__(256, (sizeof(REAL) == 4 ? 8 : 4)) k_limit(const Dev<REAL> v, int kh,
+                                                                            cudaGraphConditionalHandle h)
+{
+    if (kh == -1 && blockIdx.x == 0 && threadIdx.x == 0) advance_step(v.ctl, h);
+    kh = tile_step<ONE>(v.ctl, kh, kCtlStepOf);
     const int W = mtile_of<REAL, ONE>(v);
     const long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
     for (int w = 0; w < W; ++w) {
@@ -910,25 +941,6 @@ __global__ void __launch_bounds__(256, (sizeof(REAL) == 4 ? 8 : 4)) k_limit(cons
         int m;
         long i = split_member<ONE>(v, t, m);
         limit_cell<REAL, ONE, BIF>(v, i, m, kh);
-    }
-}
-
-// Interval loop control, run by the last kernel of a sub-step: the last
-// block to finish advances the step counter (every block has read it by
-// then) and, inside the interval graph, sets the while-condition.
-__device__ __forceinline__ void advance_step(int* ctl, cudaGraphConditionalHandle h, int set_cond)
-{
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        int done = atomicAdd(&ctl[kCtlBlocksDone], 1);
-        if (done == (int)gridDim.x - 1) {
-            ctl[kCtlBlocksDone] = 0;
-            const int next = ctl[kCtlStep] + 1;
-            ctl[kCtlStep] = next;
-            __threadfence();
-            if (set_cond) cudaGraphSetConditional(h, next < ctl[kCtlMaxSteps] ? 1u : 0u);
-        }
     }
 }
 
@@ -997,11 +1009,10 @@ __device__ __forceinline__ int levee_repartition(const Dev<REAL>& v, long li, lo
 template <typename REAL, bool ONE>
 __device__ __forceinline__ void levee_cell(const Dev<REAL>& v, long li, int m, int kh, int force_diag)
 {
-    const StepInfo st = step_info<ONE>(v.ctl, v.nsub, kh, m, force_diag);
+    const StepInfo st = step_info<ONE>(v.ctl, v.nsub, kh, m, force_diag, kCtlStepOf);
     if (!st.active) return;
-    const int k = st.k;
-    double* rdst = (k & 1) ? v.rs0 : v.rs1;
-    double* fdst = (k & 1) ? v.fs0 : v.fs1;
+    double* rdst = (st.k & 1) ? v.rs0 : v.rs1;
+    double* fdst = (st.k & 1) ? v.fs0 : v.fs1;
     const long ci = v.lci[li];
     const long cm = ix<ONE>(ci, m, v.M);
     // The cell's river and flood storage decide the regime; its depths and
@@ -1029,9 +1040,9 @@ __device__ __forceinline__ void levee_cell(const Dev<REAL>& v, long li, int m, i
 }
 
 template <typename REAL, bool ONE>
-__global__ void __launch_bounds__(256) k_levee(const Dev<REAL> v, int kh, int force_diag,
-                                               cudaGraphConditionalHandle h, int advance)
+__global__ void __launch_bounds__(256) k_levee(const Dev<REAL> v, int kh, int force_diag)
 {
+    kh = tile_step<ONE>(v.ctl, kh, kCtlStepOf);
     const int W = mtile_of<REAL, ONE>(v);
     const long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
     for (int w = 0; w < W; ++w) {
@@ -1041,13 +1052,12 @@ __global__ void __launch_bounds__(256) k_levee(const Dev<REAL> v, int kh, int fo
         const long li = split_member<ONE>(v, t, m);
         levee_cell<REAL, ONE>(v, li, m, kh, force_diag);
     }
-    if (kh == -1 && advance) advance_step(v.ctl, h, 1);
 }
 
 template <typename REAL, bool ONE, bool RES, bool LEV, bool BIF, bool BUDGET>
-__global__ void __launch_bounds__(256, CMF_STAGE_MIN_BLOCKS(REAL, ONE)) k_stage(const Dev<REAL> v, int kh, int force_diag,
-                                               cudaGraphConditionalHandle h, int set_cond)
+__global__ void __launch_bounds__(256, CMF_STAGE_MIN_BLOCKS(REAL, ONE)) k_stage(const Dev<REAL> v, int kh, int force_diag)
 {
+    kh = tile_step<ONE>(v.ctl, kh, kCtlStepOf);
     const int W = mtile_of<REAL, ONE>(v);
     if (BIF && (int)blockIdx.x >= v.cell_blocks) {
         const long t0 = (long)(blockIdx.x - v.cell_blocks) * blockDim.x + threadIdx.x;
@@ -1072,8 +1082,6 @@ __global__ void __launch_bounds__(256, CMF_STAGE_MIN_BLOCKS(REAL, ONE)) k_stage(
         }
         if (BUDGET) block_budget(bud, v.bpart, v.cell_blocks);
     }
-    // With levees, k_levee is the last kernel of the sub-step and advances.
-    if (!LEV && kh == -1) advance_step(v.ctl, h, set_cond);
 }
 
 // ---------------------------------------------------------------------------
@@ -1243,7 +1251,6 @@ __global__ void k_interval_begin(const Dev<REAL> v, double outer_seconds, int ad
         v.tsec[0] = outer_seconds;
         v.outer[0] = (REAL)outer_seconds;
         v.ctl[kCtlStep] = 0;
-        v.ctl[kCtlBlocksDone] = 0;
         if (v.rflag) {
             v.ctl[kCtlCflMax] = 0;
             v.ctl[kCtlAbort] = 0;
@@ -1379,7 +1386,7 @@ struct StatsArgs {
     double* weight;
 };
 
-// Value of a statistics variable at element t.  `after` selects the storage
+// Value of a statistics variable at element t.  `k` selects the storage
 // buffer: the state after sub-step k (k >= 0, the ping-pong destination of
 // k) or the interval state (k < 0, after k_interval_end).  Cells without a
 // levee carry protected depth == flood depth (k_stage writes that only on the
@@ -1413,8 +1420,7 @@ __device__ __forceinline__ void fold_stat(double* o, int op, double x, double dt
     else *o = (x < acc || x != x) ? x : acc;
 }
 
-// kh >= 0: host step index; kh == -1: the step that the last kernel of the
-// sub-step just finished (the device counter was advanced by it).
+// kh >= 0: host step index; kh == -1: the sub-step that k_stage has just run.
 template <typename REAL, bool ONE>
 __global__ void __launch_bounds__(256) k_stats_accumulate(const Dev<REAL> v, const StatsArgs a, int kh)
 {
@@ -1422,7 +1428,7 @@ __global__ void __launch_bounds__(256) k_stats_accumulate(const Dev<REAL> v, con
     if (t >= v.N * (long)v.M) return;
     int m;
     const long i = split_member<ONE>(v, t, m);
-    const int k = kh >= 0 ? kh : v.ctl[kCtlStep] - 1;
+    const int k = kh >= 0 ? kh : v.ctl[kCtlStepOf];
     if (k >= v.nsub[m]) return;  // member idle in this sub-step
     const double dt = (double)v.dt[m];
     if (a.need_weight && i == 0) a.weight[m] = __dadd_rn(a.weight[m], dt);

@@ -6,9 +6,8 @@
 // device->host `.item()` of the sub-step count (:122):
 //
 //   begin -> [cfl] -> plan (n, dt per member, while-condition)
-//         -> WHILE(cond) { momentum -> limit -> stage -> [levee]
-//                          (last block of the last of them: k += 1, cond = k < n)
-//                          -> [statistics] }
+//         -> WHILE(cond) { momentum -> limit (k += 1, cond = k < n) -> stage
+//                          -> [levee] -> [statistics] }
 //         -> end (storage copy-back for odd counts, current_step)
 //         -> [budget flush]
 //
@@ -455,26 +454,23 @@ int build_graph(CmfPlan* p, double T, int fixed_n)
         int kh = -1, fd = 0;
         void* a1[] = {p->dev, &kh, &fd};
         if ((rc = add_kernel(&b1, body, nullptr, 0, p->ks.momentum, grid, p->tpb, a1)) != CMF_OK) goto fail;
-        void* al[] = {p->dev, &kh};
+        void* al[] = {p->dev, &kh, &h};
         if ((rc = add_kernel(&bl, body, nullptr, 0, p->ks.limit, p->cell_blocks, p->tpb, al)) != CMF_OK)
             goto fail;
         if ((rc = add_edge(body, b1, bl)) != CMF_OK) goto fail;
-        int set = 1;
-        void* a2[] = {p->dev, &kh, &fd, &h, &set};
+        void* a2[] = {p->dev, &kh, &fd};
         if ((rc = add_kernel(&b2, body, nullptr, 0, p->ks.stage, grid, p->tpb, a2)) != CMF_OK) goto fail;
         if ((rc = add_edge(body, bl, b2)) != CMF_OK) goto fail;
         cudaGraphNode_t last = b2;
         if (p->levee_blocks > 0) {
             cudaGraphNode_t b3;
-            int adv = 1;
-            void* a3[] = {p->dev, &kh, &fd, &h, &adv};
+            void* a3[] = {p->dev, &kh, &fd};
             if ((rc = add_kernel(&b3, body, nullptr, 0, p->ks.levee, p->levee_blocks, p->tpb, a3)) != CMF_OK)
                 goto fail;
             if ((rc = add_edge(body, b2, b3)) != CMF_OK) goto fail;
             last = b3;
         }
         if (p->stats.count > 0) {
-            // after the advancing kernel: reads step counter - 1
             cudaGraphNode_t b4;
             void* a4[] = {p->dev, &p->stats, &kh};
             const int sb = ceil_div((long)v.num_catchments * v.num_members, 256);
@@ -555,11 +551,10 @@ int interval_direct(CmfPlan* p, cudaStream_t s, double T, int fixed_n)
         int kh = k, fd = 0;
         void* a1[] = {p->dev, &kh, &fd};
         if ((rc = launch(p->ks.momentum, grid, p->tpb, a1, s)) != CMF_OK) return rc;
-        void* al[] = {p->dev, &kh};
-        if ((rc = launch(p->ks.limit, p->cell_blocks, p->tpb, al, s)) != CMF_OK) return rc;
         cudaGraphConditionalHandle h = 0;
-        int set = 0;
-        void* a2[] = {p->dev, &kh, &fd, &h, &set};
+        void* al[] = {p->dev, &kh, &h};
+        if ((rc = launch(p->ks.limit, p->cell_blocks, p->tpb, al, s)) != CMF_OK) return rc;
+        void* a2[] = {p->dev, &kh, &fd};
         if ((rc = launch(p->ks.stage, grid, p->tpb, a2, s)) != CMF_OK) return rc;
         if (p->levee_blocks > 0) {
             if ((rc = launch(p->ks.levee, p->levee_blocks, p->tpb, a2, s)) != CMF_OK) return rc;
@@ -904,11 +899,10 @@ int cmf_phase_stage(CmfPlan* p, void* stream, int diag)
     cudaStream_t s = (cudaStream_t)stream;
     int kh = -2, fd = diag ? 1 : 2;
     cudaGraphConditionalHandle h = 0;
-    int set = 0;
-    void* al[] = {p->dev, &kh};
+    void* al[] = {p->dev, &kh, &h};
     int rc = launch(p->ks.limit, p->cell_blocks, p->tpb, al, s);
     if (rc != CMF_OK) return rc;
-    void* args[] = {p->dev, &kh, &fd, &h, &set};
+    void* args[] = {p->dev, &kh, &fd};
     rc = launch(p->ks.stage, p->cell_blocks + p->path_blocks, p->tpb, args, s);
     if (rc != CMF_OK) return rc;
     if (p->levee_blocks > 0) {
@@ -971,20 +965,17 @@ int cmf_launch_substep(CmfPlan* p, void* stream, int32_t k, int part)
         return launch(p->ks.momentum, grid, p->tpb, a1, s);
     }
     if (part == CMF_PART_LIMIT) {
-        void* al[] = {p->dev, &kh};
+        cudaGraphConditionalHandle h = 0;
+        void* al[] = {p->dev, &kh, &h};
         return launch(p->ks.limit, p->cell_blocks, p->tpb, al, s);
     }
     if (part == CMF_PART_STAGE) {
-        cudaGraphConditionalHandle h = 0;
-        int set = 0;
-        void* a2[] = {p->dev, &kh, &fd, &h, &set};
+        void* a2[] = {p->dev, &kh, &fd};
         return launch(p->ks.stage, grid, p->tpb, a2, s);
     }
     if (part == CMF_PART_LEVEE) {
         if (p->levee_blocks == 0) return CMF_OK;
-        cudaGraphConditionalHandle h = 0;
-        int set = 0;
-        void* a3[] = {p->dev, &kh, &fd, &h, &set};
+        void* a3[] = {p->dev, &kh, &fd};
         return launch(p->ks.levee, p->levee_blocks, p->tpb, a3, s);
     }
     if (part == CMF_PART_END) {
