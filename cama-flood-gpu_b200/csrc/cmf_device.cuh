@@ -675,6 +675,16 @@ struct CellProfile {
         ca = v->ca[i];
         loaded = true;
     }
+    // Starts the row and the area of a wet cell on their way to L2, where the
+    // row is walked from memory: the walk begins a DRAM round trip after the
+    // cell's other loads (6M full physics, k_stage: 228 -> 220 us; for dry cells
+    // too it was 224).
+    __device__ void prefetch(bool wet) const
+    {
+        if (kRegs || !wet) return;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(v->tbl + i * (long)v->K));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(v->ca + i));
+    }
     __device__ bool in_regs() const { return REGS && v->K == kRowRegs; }
     __device__ REAL area()
     {
@@ -742,13 +752,12 @@ __device__ __forceinline__ double path_net(REAL raw, int e, REAL lr_i, REAL lr_o
     return (e & 1) ? (double)(-net) : (double)net;
 }
 
-// Bifurcation net outflow of cell i, whose limit rate is lr_i
+// Bifurcation net outflow of the cell with path ends [b0, b1) and limit rate lr_i
 // (bifurcation.cu:131-156 gathered over the cell's path ends).
 template <typename REAL, bool ONE>
-__device__ __forceinline__ double path_net_of(const Dev<REAL>& v, long i, int m, REAL lr_i)
+__device__ __forceinline__ double path_net_of(const Dev<REAL>& v, int b0, int b1, int m, REAL lr_i)
 {
     double gb = 0.0;
-    const int b0 = v.bptr[i], b1 = v.bptr[i + 1];
     for (int b = b0; b < b1; ++b) {
         const int e = v.bpaths[b];
         const int p = e >> 1;
@@ -804,6 +813,19 @@ __device__ __forceinline__ void stage_cell(const Dev<REAL>& v, long i, int m, in
     prof.i = i;
     prof.loaded = false;
     if (prof.in_regs() && fsto > 0.0) prof.load();
+    prof.prefetch(fsto > 0.0);
+    // Chains that end a single member's sub-step, begun before the gather: the
+    // downstream cell of a backward flux, whose rate it takes, and the cell's
+    // path ends.  (With members, a warp's lanes share the cell, and the held
+    // registers cost more: 130 -> 140 us.)
+    const bool back = !mouth && (qr < (REAL)0.0 || qf < (REAL)0.0);
+    const bool ends = BIF && (fl & CMF_CELL_BIFURCATION);
+    int dn_i = 0, b0 = 0, b1 = 0;
+    if (ONE && ends) {
+        b0 = v.bptr[i];
+        b1 = v.bptr[i + 1];
+    }
+    if (ONE && back) dn_i = v.dn[i];
 
     // upstream inflow: gather the limited fluxes of the upstream cells, in
     // range order, child_unroll independent loads at a time
@@ -835,13 +857,18 @@ __device__ __forceinline__ void stage_cell(const Dev<REAL>& v, long i, int m, in
 
     // own limited flux (the downstream rate is needed only for negative flux)
     REAL lr_dn = lr_i;
-    if (!mouth && (qr < (REAL)0.0 || qf < (REAL)0.0))
-        lr_dn = v.lrs[ix<ONE>(v.dn[i], m, M)];
+    if (back) lr_dn = v.lrs[ix<ONE>(ONE ? dn_i : v.dn[i], m, M)];
     const REAL rout = (qr >= (REAL)0.0) ? qr * lr_i : qr * lr_dn;
     const REAL fout = (qf >= (REAL)0.0) ? qf * lr_i : qf * lr_dn;
 
     double gb = 0.0;
-    if (BIF && (fl & CMF_CELL_BIFURCATION)) gb = path_net_of<REAL, ONE>(v, i, m, lr_i);
+    if (ends) {
+        if (!ONE) {
+            b0 = v.bptr[i];
+            b1 = v.bptr[i + 1];
+        }
+        gb = path_net_of<REAL, ONE>(v, b0, b1, m, lr_i);
+    }
 
     // continuity and flood stage; levee cells are re-partitioned afterwards
     // by k_levee, which conserves river + flood + protected storage, so the
