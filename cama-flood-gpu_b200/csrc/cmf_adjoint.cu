@@ -31,10 +31,10 @@
 //   kr_limit       limit-rate and outgoing-storage adjoints;
 //   kr_momentum    local-inertial momentum reversed per cell;
 //   kr_dam         reservoir release and the dam-upstream kinematic flow
-//                  reversed for the dam cells (trailing blocks of the
+//                  reversed for the dam cells (leading blocks of the
 //                  kr_momentum launch, applied one sub-step later);
 //   kr_path        path momentum reversed, one thread per path and input
-//                  direction (trailing blocks of the kr_momentum launch).
+//                  direction (leading blocks of the kr_momentum launch).
 //
 // The long scalar branches -- reservoir release, dam-upstream kinematic flow,
 // path momentum with its limiter, levee re-partition -- are templates on the
@@ -605,8 +605,9 @@ __device__ __forceinline__ double store_eval(double rsto, double fsto, double pr
 __global__ void __launch_bounds__(kBlock, CMF_ADJ_MIN_BLOCKS) ka_momentum(const Ctx c, double* X, double* Y,
                                                       const double* runoff, double dt)
 {
-    if ((int)blockIdx.x >= c.grid_cells) {
-        const long p = (long)(blockIdx.x - c.grid_cells) * blockDim.x + threadIdx.x;
+    const int block = (int)blockIdx.x - c.grid_paths;  // the paths' blocks come first
+    if (block < 0) {
+        const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
         if (p >= c.P) return;
         double in[6 + 2 * kMaxLevels], blim[kMaxLevels], bcsd_new[kMaxLevels], bsum;
         path_inputs(c, X, p, in);
@@ -623,7 +624,7 @@ __global__ void __launch_bounds__(kBlock, CMF_ADJ_MIN_BLOCKS) ka_momentum(const 
         braw_of(c, X)[p] = raw;
         return;
     }
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long i = (long)block * blockDim.x + threadIdx.x;
     if (i >= c.N) return;
     Mom m;
     mom_eval(c, X, i, dt, m);
@@ -1118,7 +1119,7 @@ __global__ void __launch_bounds__(kBlock) kr_limit(const Ctx c, const double* X,
 // them, so the primal part of the evaluation (roots, divisions, branches)
 // runs once per kPathLanes directions; it writes each direction's adjoint:
 // lambda_k of the path state, or an end-state adjoint left for the end cell.
-// Runs as the trailing blocks of the kr_momentum launch: it reads the tape,
+// Runs as the leading blocks of the kr_momentum launch: it reads the tape,
 // the outgoing-storage adjoint of kr_limit and the path buffers of
 // kr_stage_path, and writes only the path lambdas and the path-end buffer,
 // none of which the momentum or dam reverse touches.  Two lanes: wider
@@ -1401,10 +1402,13 @@ __global__ void __launch_bounds__(kBlock, CMF_ADJ_MIN_BLOCKS) kr_momentum(const 
                                                       const double* runoff, double dt, Adj a)
 {
     pdl_begin();
-    if ((int)blockIdx.x >= c.grid_cells) {
-        // trailing blocks: path direction threads, then dam direction threads
-        const long b = (long)blockIdx.x - c.grid_cells;
-        const long pb = c.bif ? (c.P * path_reverse_threads(c.P, c.L) + kBlock - 1) / kBlock : 0;
+    // Leading blocks: path direction threads, then dam direction threads.  Their
+    // chains are the longest; as trailing blocks they stood alone at the end of
+    // the grid (250k full physics: 60 -> 51 us; ka_momentum 25 -> 19).
+    const long pb = c.bif ? (c.P * path_reverse_threads(c.P, c.L) + kBlock - 1) / kBlock : 0;
+    const long lead = pb + ((c.res && c.ND > 0) ? (c.ND * kDamDirs + kBlock - 1) / kBlock : 0);
+    if ((long)blockIdx.x < lead) {
+        const long b = (long)blockIdx.x;
         if (b < pb) {
             if (CMF_ADJ_PATH_HAND) path_reverse_hand(c, X, dt, a, b * blockDim.x + threadIdx.x);
             else path_reverse(c, X, dt, a, b * blockDim.x + threadIdx.x);
@@ -1414,7 +1418,7 @@ __global__ void __launch_bounds__(kBlock, CMF_ADJ_MIN_BLOCKS) kr_momentum(const 
     }
     const long N = c.N;
     double* lam = a.lam;
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long i = ((long)blockIdx.x - lead) * blockDim.x + threadIdx.x;
     if (i >= N) return;
     Mom m;
     mom_eval(c, X, i, dt, m);
@@ -1568,7 +1572,7 @@ __device__ __forceinline__ void flux_bars(const Ctx& c, const double* X, const A
 }
 
 // Reservoir release and dam-upstream kinematic flow reversed (kr_dam), one
-// thread per dam cell and input direction (one dual pass each), as trailing
+// thread per dam cell and input direction (one dual pass each), as leading
 // blocks of the kr_momentum launch.  kr_momentum writes the same cells'
 // lambdas, so these adjoints go to the dam scratch instead and apply_pending
 // adds them at the start of the earlier sub-step (before anything reads those
@@ -1854,7 +1858,7 @@ int cmf_adj_reverse(CmfAdjPlan* plan, void* stream, const double* tape, int num_
         launch_dep(kr_stage, c.grid_cells, s, c, X, runoff, dt, a);
         if (c.bif) launch_dep(kr_stage_path, c.grid_paths, s, c, X, a);
         launch_dep(kr_limit, c.grid_cells, s, c, X, dt, a);
-        // cells, then the path and dam direction threads in trailing blocks
+        // the path and dam direction threads in leading blocks, then the cells
         const int path_blocks = c.bif ? (int)((c.P * path_reverse_threads(c.P, c.L) + kBlock - 1) / kBlock) : 0;
         const int dam_blocks = (c.res && c.ND > 0) ? (int)((c.ND * kDamDirs + kBlock - 1) / kBlock) : 0;
         launch_dep(kr_momentum, c.grid_cells + path_blocks + dam_blocks, s, c, X, runoff, dt, a);
