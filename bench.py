@@ -1036,6 +1036,8 @@ def run_ours(args) -> None:
     substeps = int(counts[args.warmup:].sum().item())
     per_sub = 4 if Lv > 0 else 3                 # momentum, limit, stage (+ levee)
     launches = 4 * args.steps + per_sub * substeps   # + begin, cfl, plan, end per interval
+    if model.resident_tiles:                     # begin and the resident kernel
+        launches = 2 * args.steps
     t = torch.tensor([ms], dtype=torch.float64, device=device)
     w = torch.tensor([N * substeps], dtype=torch.float64, device=device)
     if world > 1:

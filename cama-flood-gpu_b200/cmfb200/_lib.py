@@ -170,6 +170,8 @@ def lib() -> ctypes.CDLL:
     h.cmf_plan_destroy.argtypes = [_P]
     h.cmf_plan_set_member_tile.restype = ctypes.c_int
     h.cmf_plan_set_member_tile.argtypes = [_P, _I32]
+    h.cmf_plan_resident_tiles.restype = ctypes.c_int
+    h.cmf_plan_resident_tiles.argtypes = [_P]
     h.cmf_plan_set_persistent.restype = ctypes.c_int
     h.cmf_plan_set_persistent.argtypes = [_P, ctypes.c_int]
     h.cmf_probe_barrier_timeout.restype = ctypes.c_int

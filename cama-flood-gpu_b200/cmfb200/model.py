@@ -805,6 +805,13 @@ class CaMaFlood:
         _lib.check(rc, "plan_set_persistent")
         self.persistent = bool(on)
 
+    @property
+    def resident_tiles(self) -> int:
+        """Tiles of the resident interval kernel that step_advance takes (a
+        network whose state fits the SMs' shared memory: one member, no
+        budget); 0 where it takes the interval graph or another form."""
+        return int(_lib.lib().cmf_plan_resident_tiles(self._plan))
+
     def autotune_block_size(self, candidates=None, sub_steps: int = 6,
                             cache_path: Optional[str] = None, tile_candidates=None) -> dict:
         """Measure the candidate CTA sizes (and, with several members, member

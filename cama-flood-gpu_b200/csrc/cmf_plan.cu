@@ -1028,6 +1028,11 @@ int cmf_plan_set_persistent(CmfPlan* p, int enable)
     return CMF_OK;
 }
 
+int cmf_plan_resident_tiles(const CmfPlan* p)
+{
+    return p && p->graph_enabled && !p->persistent ? p->resident_tiles : 0;
+}
+
 int cmf_probe_barrier_timeout(void* stream, int32_t* control, int32_t* status, int32_t timeout_us)
 {
     if (!control || !status || timeout_us <= 0 || timeout_us > 1000000) return CMF_ERR_ARG;

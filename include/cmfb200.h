@@ -236,6 +236,12 @@ void cmf_plan_destroy(CmfPlan* plan);
  * CMF_STATUS_SYNC_TIMEOUT and ends the interval.  enable == 0 returns to the
  * interval graph. */
 int cmf_plan_set_persistent(CmfPlan* plan, int enable);
+/* Tiles of the resident interval kernel that cmf_step_interval takes for this
+ * plan: one member without budget whose state fits the SMs' shared memory runs
+ * a whole interval in one cooperative launch after the prologue (the interval
+ * graph inside a stream capture).  0: the plan takes another form. */
+int cmf_plan_resident_tiles(const CmfPlan* plan);
+
 /* Test of the persistent kernel's failure path (no counterpart in the
  * reference): launches, cooperatively, two blocks that meet at a grid barrier
  * waiting for one arrival more than they make, so each wait gives up after

@@ -21,6 +21,7 @@ SAVED = {"mean": ["total_outflow", "flood_fraction"], "max": ["river_depth", "ri
 
 def _run(net, graph, days=2, fixed=None, saved=None, **kw):
     m = P.model_for(net, use_cuda_graph=graph, variables_to_save=saved, **kw)
+    assert (m.resident_tiles > 0) == graph
     counts = []
     for d in range(days):
         m.set_inputs(torch.as_tensor(m.to_model_order(20.0 * syn.daily_runoff(net, d))).cuda())
@@ -57,9 +58,9 @@ def test_resident_small_networks(n, device):
     _same(syn.generate(syn.NetworkSpec(n, seed=3)))
 
 
-@pytest.mark.parametrize("n, precision", [(45_001, "float64"), (150_001, "float32"), (300_011, "float32")])
+@pytest.mark.parametrize("n, precision", [(45_001, "float64"), (150_001, "float32"), (250_007, "float32")])
 def test_resident_several_cells_per_thread(n, precision, device):
-    """Rows in shared memory, several cells per thread, and (300k) rows in L2."""
+    """Rows in shared memory, several cells per thread, and (250k) rows in L2."""
     net = syn.generate(syn.NetworkSpec(n, seed=5, bifurcation_paths=n // 30, levee_fraction=0.2,
                                        reservoirs=n // 700))
     _same(net, precision=precision, days=1, fixed=30)
@@ -77,3 +78,14 @@ def test_resident_sub_step_cap_and_dt_cap(device):
     assert int(m.sub_step_counts()[0].item()) == 3
     with pytest.raises(RuntimeError):
         m.check_status()
+
+
+def test_resident_is_left_to_what_it_runs(device):
+    """Members, the budget, the persistent kernel and a network beyond the
+    SMs' shared memory take their own forms."""
+    net = P.make_network("plain", n=2000)
+    assert P.model_for(net).resident_tiles == 16
+    assert P.model_for(net, budget=True).resident_tiles == 0
+    assert P.model_for(net, persistent=True).resident_tiles == 0
+    assert P.model_for(net, num_members=2).resident_tiles == 0
+    assert P.model_for(syn.generate(syn.NetworkSpec(400_000, seed=1))).resident_tiles == 0
