@@ -584,11 +584,11 @@ int interval_direct(CmfPlan* p, cudaStream_t s, double T, int fixed_n)
 // Tiles of the resident kernel for this plan's network, if it fits: one tile
 // per SM, as many cells as spread the network over the SMs, and the
 // floodplain rows in shared memory too where they find room.  It is taken
-// wherever it fits, because it was the faster form at every such size: a daily
-// interval through the interval graph and through this kernel, us per
-// sub-step: 60k plain 27.2 / 7.0, 250k full physics 45.7 / 21.2, 100k full
-// physics with two statistics 40.3 / 13.8, 30k full physics fp64 37.4 / 16.7;
-// an hour of 4k full physics 32.1 / 11.2.
+// wherever it fits, because it was the faster form at every such size.  Through
+// the interval graph and through this kernel: an hour of 4k full physics 854 /
+// 345 us; a day of 60k plain 17.1 / 5.5 ms, of 100k full physics with two
+// statistics 25.4 / 9.6 ms, of 250k full physics 35.3 / 17.1 ms, of 30k full
+// physics in fp64 26.6 / 13.9 ms.
 int plan_resident(CmfPlan* p, const Layout& L)
 {
     p->resident_tiles = 0;
@@ -613,6 +613,9 @@ int plan_resident(CmfPlan* p, const Layout& L)
     ResidentArgs& a = p->resident;
     std::memset(&a, 0, sizeof(a));
     a.tile = tile;
+    const int real = p->fp64 ? 8 : 4;
+    resident_layout(a, real, v.num_flood_levels, v.num_bifurcation_levels, false);
+    if (a.bytes > room) return CMF_OK;  // the cells alone do not fit
     char* ws = (char*)v.workspace;
     void* args[] = {p->dev, &tile};
     const void* scan = p->fp64 ? (const void*)k_resident_scan<double> : (const void*)k_resident_scan<float>;
@@ -620,7 +623,6 @@ int plan_resident(CmfPlan* p, const Layout& L)
     if ((rc = check_cuda(cudaMemcpy(&a.most, (int*)(ws + L.ctl) + kCtlTileMax, sizeof(a.most),
                                     cudaMemcpyDeviceToHost))) != CMF_OK)
         return rc;
-    const int real = p->fp64 ? 8 : 4;
     resident_layout(a, real, v.num_flood_levels, v.num_bifurcation_levels, true);
     if (a.bytes > room) resident_layout(a, real, v.num_flood_levels, v.num_bifurcation_levels, false);
     if (a.bytes > room) return CMF_OK;

@@ -89,3 +89,25 @@ def test_resident_is_left_to_what_it_runs(device):
     assert P.model_for(net, persistent=True).resident_tiles == 0
     assert P.model_for(net, num_members=2).resident_tiles == 0
     assert P.model_for(syn.generate(syn.NetworkSpec(400_000, seed=1))).resident_tiles == 0
+
+
+def test_resident_models_on_streams_of_their_own(device):
+    """Two models, each on its own stream, one of high priority, their intervals
+    in flight together: each equals its own run on one stream."""
+    nets = [P.make_network("full", n=40_000, seed=2), P.make_network("bif", n=23_000, seed=6)]
+    alone = [_run(net, True, days=3)[0] for net in nets]
+    models = [P.model_for(net) for net in nets]
+    runoff = [[torch.as_tensor(m.to_model_order(20.0 * syn.daily_runoff(net, d))).cuda() for d in range(3)]
+              for m, net in zip(models, nets)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(priority=0), torch.cuda.Stream(priority=-1)]
+    for d in range(3):
+        for m, s, r in zip(models, streams, runoff):
+            with torch.cuda.stream(s):
+                m.set_inputs(r[d])
+                m.step_advance()
+    torch.cuda.synchronize()
+    for m, a in zip(models, alone):
+        m.check_status()
+        for k, v in m.state_tensors().items():
+            np.testing.assert_array_equal(v.cpu().numpy(), a[k], err_msg=k)
