@@ -795,9 +795,10 @@ class CaMaFlood:
     def set_persistent(self, on: bool = True) -> None:
         """Run each interval's sub-steps in one persistent cooperative kernel
         (grid-wide barriers between the phases) instead of the interval
-        graph; the results are the same.  It pays on small networks, where a
-        sub-step is a few microseconds of work.  One member, no budget and no
-        output statistics; raises otherwise."""
+        graph or the resident kernel; the results are the same.  No measured
+        network is faster with it (small ones run in the resident kernel by
+        themselves, large ones are faster through the graph).  One member, no
+        budget and no output statistics; raises otherwise."""
         rc = _lib.lib().cmf_plan_set_persistent(self._plan, 1 if on else 0)
         if rc == _lib.CMF_ERR_UNSUPPORTED:
             raise ValueError("the persistent interval kernel runs one member without budget or "

@@ -1122,9 +1122,9 @@ __global__ void __launch_bounds__(256, CMF_STAGE_MIN_BLOCKS(REAL, ONE)) k_stage(
 // grid-wide barrier after each phase (momentum, limit rate, stage, levee),
 // where the interval graph has a kernel boundary; the per-element work is
 // the same device functions the four sub-step kernels call, with the step
-// index passed explicitly.  On small networks the sub-step is a few
-// microseconds of work, and a barrier costs less than a graph's kernel
-// boundary.
+// index passed explicitly.  Kept for the callers that ask for it: networks that
+// fit the SMs' shared memory are faster in the resident kernel
+// (cmf_resident.cuh), larger ones through the interval graph.
 //
 // The barrier counts arrivals on a monotone 64-bit counter (reset by
 // k_interval_plan): the b-th barrier of the launch completes when the counter
