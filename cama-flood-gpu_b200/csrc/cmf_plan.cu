@@ -581,7 +581,8 @@ int interval_direct(CmfPlan* p, cudaStream_t s, double T, int fixed_n)
     return CMF_OK;
 }
 
-// Tiles of the resident kernel for this plan's network, if it fits: one tile
+// Tiles of the resident kernel for this plan's network, if it fits and its
+// lists are in the form that the kernel indexes by (k_resident_scan): one tile
 // per SM, as many cells as spread the network over the SMs, and the
 // floodplain rows in shared memory too where they find room.  It is taken
 // wherever it fits, because it was the faster form at every such size.  Through
@@ -620,9 +621,13 @@ int plan_resident(CmfPlan* p, const Layout& L)
     void* args[] = {p->dev, &tile};
     const void* scan = p->fp64 ? (const void*)k_resident_scan<double> : (const void*)k_resident_scan<float>;
     if ((rc = launch(scan, tiles, 256, args, 0)) != CMF_OK) return rc;
-    if ((rc = check_cuda(cudaMemcpy(&a.most, (int*)(ws + L.ctl) + kCtlTileMax, sizeof(a.most),
+    TileScan found;
+    static_assert(kCtlTileMax + sizeof(TileScan) / sizeof(int) <= 16, "the control words end here");
+    if ((rc = check_cuda(cudaMemcpy(&found, (int*)(ws + L.ctl) + kCtlTileMax, sizeof(found),
                                     cudaMemcpyDeviceToHost))) != CMF_OK)
         return rc;
+    if (found.irregular) return CMF_OK;
+    a.most = found.most;
     resident_layout(a, real, v.num_flood_levels, v.num_bifurcation_levels, true);
     if (a.bytes > room) resident_layout(a, real, v.num_flood_levels, v.num_bifurcation_levels, false);
     if (a.bytes > room) return CMF_OK;

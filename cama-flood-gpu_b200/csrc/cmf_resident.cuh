@@ -706,35 +706,54 @@ __device__ __forceinline__ int first_at_least(const int* list, int n, int x)
     return lo;
 }
 
-// TileCounts of every tile (one block each), their maxima into
-// ctl[kCtlTileMax ..]; once per plan.
+// What k_resident_scan leaves at ctl[kCtlTileMax ..].
+struct TileScan {
+    TileCounts most;  // maxima over the tiles
+    int irregular;    // not 0: the view's lists are not in the form below
+};
+
+// TileCounts of every tile (one block each) and the form of the lists that
+// k_resident indexes by, once per plan.  A levee of the tile is found by
+// bisection of the levee list and writes its cell's slot, so the list has to be
+// strictly ascending, in range, and exactly the cells flagged as levee cells;
+// a path end elsewhere answers only if its cell is flagged for bifurcation.
+// The sub-step kernels ask for neither (levee_slot maps any order).
 template <typename REAL>
 __global__ void __launch_bounds__(256) k_resident_scan(const Dev<REAL> v, int tile)
 {
-    __shared__ int own, dams, lo, hi;
+    __shared__ int own, dams, levees, bad, lo, hi;
     const int t0 = blockIdx.x * tile, t1 = min(t0 + tile, (int)v.N);
-    if (threadIdx.x == 0) { own = dams = hi = 0; lo = INT32_MAX; }
+    if (threadIdx.x == 0) { own = dams = levees = bad = hi = 0; lo = INT32_MAX; }
     __syncthreads();
     for (int i = t0 + threadIdx.x; i < t1; i += blockDim.x) {
         const int c0 = v.up[i], c1 = upstream_end(v, (long)i);
+        const uint8_t fl = v.flags[i];
         if (c0 < c1 && c1 > t1) {
             atomicMin(&lo, max(c0, t1));
             atomicMax(&hi, c1);
         }
-        if ((v.features & CMF_FEAT_RESERVOIR) && (v.flags[i] & CMF_CELL_RESERVOIR)) atomicAdd(&dams, 1);
+        if ((v.features & CMF_FEAT_RESERVOIR) && (fl & CMF_CELL_RESERVOIR)) atomicAdd(&dams, 1);
+        if ((v.features & CMF_FEAT_LEVEE) && (fl & CMF_CELL_LEVEE)) atomicAdd(&levees, 1);
+        if ((v.features & CMF_FEAT_BIFURCATION) && v.bptr[i] < v.bptr[i + 1] && !(fl & CMF_CELL_BIFURCATION)) bad = 1;
     }
     if (v.features & CMF_FEAT_BIFURCATION)
         for (int x = v.bptr[t0] + threadIdx.x; x < v.bptr[t1]; x += blockDim.x)
             if (!(v.bpaths[x] & 1)) atomicAdd(&own, 1);
+    for (long l = (long)blockIdx.x * blockDim.x + threadIdx.x; l < v.NLV; l += (long)gridDim.x * blockDim.x) {
+        const int c = v.lci[l];
+        if (c < 0 || c >= v.N || (l > 0 && v.lci[l - 1] >= c) || !(v.flags[c] & CMF_CELL_LEVEE)) bad = 1;
+    }
     __syncthreads();
     if (threadIdx.x != 0) return;
     int* most = v.ctl + kCtlTileMax;
     if (v.features & CMF_FEAT_BIFURCATION) atomicMax(most, v.bptr[t1] - v.bptr[t0]);
     atomicMax(most + 1, own);
-    if (v.NLV > 0)
-        atomicMax(most + 2, first_at_least(v.lci, (int)v.NLV, t1) - first_at_least(v.lci, (int)v.NLV, t0));
+    int listed = 0;
+    if (v.NLV > 0) listed = first_at_least(v.lci, (int)v.NLV, t1) - first_at_least(v.lci, (int)v.NLV, t0);
+    atomicMax(most + 2, listed);
     atomicMax(most + 3, dams);
     if (hi > 0) atomicMax(most + 4, hi - lo);
+    if (bad || levees != listed) atomicMax(most + 5, 1);
 }
 
 template <typename REAL, bool RES, bool LEV, bool BIF>
@@ -760,7 +779,7 @@ k_resident(const Dev<REAL> v, const StatsArgs stats, const ResidentArgs a)
     const int ends0 = BIF ? v.bptr[t.t0] : 0;
     for (int j = tid; j < t.count; j += nthr) {
         const int i = t.t0 + j;
-        uint8_t fl = v.flags[i];
+        uint8_t fl = v.flags[i] & ~(kRemoteDown | kRemoteUp);  // no CMF_CELL_* bits: a caller may use them
         const int dn = v.dn[i], c0 = v.up[i], c1 = upstream_end(v, (long)i);
         t.dn[j] = dn;
         t.c0[j] = c0;

@@ -1,0 +1,84 @@
+"""Lists of a view in a form that the resident interval kernel cannot index by:
+a levee list that is not ascending, a levee cell that no levee lists, a path end
+in a cell that is not flagged for bifurcation.  The plan leaves such a view to
+the interval graph, whose results are those of the same view with the sub-step
+kernels launched one by one.  Flag bits that the library does not define change
+nothing."""
+import numpy as np
+import pytest
+import torch
+
+from cmfb200 import _lib, synthetic as syn
+
+import parity as P
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(m, net, days=2):
+    for d in range(days):
+        m.set_inputs(torch.as_tensor(m.to_model_order(20.0 * syn.daily_runoff(net, d))).cuda())
+        m.step_advance()
+    torch.cuda.synchronize()
+    m.check_status()
+    return {k: v.cpu().numpy() for k, v in m.state_tensors().items()}
+
+
+def _same(a, b):
+    for k in a:
+        np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+
+
+def _shuffled_levees(m):
+    """The same levees listed in another order."""
+    lm = m.levee
+    perm = torch.randperm(lm.num_levees, generator=torch.Generator().manual_seed(4)).to(m.device)
+    for k in ("levee_catchment_idx", "levee_crown_height", "levee_fraction", "levee_base_height"):
+        getattr(lm, k).copy_(getattr(lm, k)[perm])
+    m.base.levee_slot[lm.levee_catchment_idx.long()] = torch.arange(lm.num_levees, dtype=torch.int32,
+                                                                    device=m.device)
+
+
+def _unlisted_levee(m):
+    """The last levee taken off the list, its cell still flagged."""
+    m.base.levee_slot[m.levee.levee_catchment_idx[-1].long()] = -1
+    m.levee.num_levees -= 1
+
+
+def _unflagged_path_ends(m):
+    cells = m.bifurcation.bifurcation_downstream_idx[:20].long()
+    m.base.cell_flags[cells] &= 255 - _lib.CELL_BIFURCATION
+
+
+@pytest.mark.parametrize("precision", ["float32", "float64"])
+def test_levees_in_any_order(precision, device):
+    net = P.make_network("full", n=9001)
+    plain = P.model_for(net, precision=precision)
+    assert plain.resident_tiles > 0
+    mixed = P.model_for(net, precision=precision)
+    _shuffled_levees(mixed)
+    mixed._rebuild_plan(mixed.block_size)
+    assert mixed.resident_tiles == 0
+    _same(_run(plain, net), _run(mixed, net))
+
+
+@pytest.mark.parametrize("change", [_unlisted_levee, _unflagged_path_ends])
+def test_lists_that_disagree_with_the_flags(change, device):
+    net = P.make_network("full", n=5000)
+    runs = []
+    for graph in (True, False):
+        m = P.model_for(net, use_cuda_graph=graph)
+        change(m)
+        m._rebuild_plan(m.block_size)
+        assert m.resident_tiles == 0
+        runs.append(_run(m, net))
+    _same(*runs)
+
+
+def test_undefined_flag_bits_are_ignored(device):
+    net = P.make_network("full", n=5000)
+    plain, marked = P.model_for(net), P.model_for(net)
+    marked.base.cell_flags |= 192
+    marked._rebuild_plan(marked.block_size)
+    assert marked.resident_tiles > 0
+    _same(_run(plain, net), _run(marked, net))
