@@ -801,9 +801,14 @@ int cmf_plan_create(const CmfView* view, CmfPlan** out)
         p->ks = pick_one<float>(p->one, res, lev, bif, bud);
         fill_dev<float>(p, L, true);
     }
-    // clear the control words and budget partials once
+    // The plan's own work runs on the legacy stream, which does not wait for the
+    // caller's non-blocking streams, nor they for it: the topology and the
+    // workspace's first fill may still be on their way, and the first interval
+    // may come on any stream.  So the device is idle before it and after it.
+    // Clear the control words and budget partials once.
     char* ws = (char*)view->workspace;
-    if ((rc = check_cuda(cudaMemset(ws + L.bpart, 0, L.tsec + 8 - L.bpart))) != CMF_OK) {
+    if ((rc = check_cuda(cudaDeviceSynchronize())) != CMF_OK ||
+        (rc = check_cuda(cudaMemset(ws + L.bpart, 0, L.tsec + 8 - L.bpart))) != CMF_OK) {
         delete p;
         return rc;
     }
@@ -812,14 +817,12 @@ int cmf_plan_create(const CmfView* view, CmfPlan** out)
         // shared river geometry, the levees' marks
         void* args[] = {p->dev};
         const void* fn = p->fp64 ? (const void*)k_levee_pack<double> : (const void*)k_levee_pack<float>;
-        rc = launch(fn, ceil_div((long)view->num_levees, 256), 256, args, 0);
-        if (rc == CMF_OK) rc = check_cuda(cudaDeviceSynchronize());
-        if (rc != CMF_OK) {
+        if ((rc = launch(fn, ceil_div((long)view->num_levees, 256), 256, args, 0)) != CMF_OK) {
             delete p;
             return rc;
         }
     }
-    if ((rc = plan_resident(p, L)) != CMF_OK) {
+    if ((rc = plan_resident(p, L)) != CMF_OK || (rc = check_cuda(cudaDeviceSynchronize())) != CMF_OK) {
         delete p;
         return rc;
     }

@@ -215,7 +215,10 @@ size_t cmf_view_size(void);
 int cmf_workspace_size(const CmfView* view, size_t* bytes);
 /* Validate the view and bind a plan to its pointers (cmfgpu phys dispatch:
  * BackendRegistry(...).selected binding by parameter name,
- * cmfgpu/phys/outflow.py:51-60).  With levees, the plan copies each levee
+ * cmfgpu/phys/outflow.py:51-60).  Reads the topology, the flags and the lists,
+ * which stay as they are while the plan lives: it waits for the device before
+ * it does (they may come from any stream) and again before it returns, so it
+ * cannot be called inside a stream capture.  With levees, the plan copies each levee
  * cell's floodplain row and (when not member-batched) river height, width
  * and length into the workspace once, synchronously, and with that shared
  * geometry computes each levee's marks: the storages at which its regimes
