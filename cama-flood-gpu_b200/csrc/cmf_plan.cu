@@ -337,6 +337,33 @@ int launch(const void* fn, int grid, int block, void** args, cudaStream_t s)
     return check_cuda(cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, s));
 }
 
+// The device that holds p current for a scope: a plan's own work runs where its
+// tensors are, whichever device the caller has current.
+class OnDeviceOf {
+public:
+    explicit OnDeviceOf(const void* p)
+    {
+        cudaPointerAttributes at;
+        if ((rc_ = check_cuda(cudaGetDevice(&before_))) != CMF_OK) return;
+        if ((rc_ = check_cuda(cudaPointerGetAttributes(&at, p))) != CMF_OK) return;
+        if (at.type == cudaMemoryTypeDevice && at.device != before_) {
+            if ((rc_ = check_cuda(cudaSetDevice(at.device))) != CMF_OK) return;
+            moved_ = true;
+        }
+    }
+    ~OnDeviceOf()
+    {
+        if (moved_) cudaSetDevice(before_);
+    }
+    OnDeviceOf(const OnDeviceOf&) = delete;
+    OnDeviceOf& operator=(const OnDeviceOf&) = delete;
+    int status() const { return rc_; }
+
+private:
+    int before_ = 0, rc_ = CMF_OK;
+    bool moved_ = false;
+};
+
 int validate(const CmfView* v)
 {
     if (!v) return CMF_ERR_ARG;
@@ -772,6 +799,8 @@ int cmf_plan_create(const CmfView* view, CmfPlan** out)
     size_t need = 0;
     cmf_workspace_size(view, &need);
     if (view->workspace_bytes < need) return CMF_ERR_ARG;
+    const OnDeviceOf device(view->workspace);
+    if (device.status() != CMF_OK) return device.status();
     CmfPlan* p = new (std::nothrow) CmfPlan;
     if (!p) return CMF_ERR_ARG;
     std::memset((void*)p, 0, sizeof(CmfPlan));
