@@ -838,7 +838,7 @@ class CaMaFlood:
         if s & _lib.STATUS_SUBSTEP_CAP:
             raise RuntimeError("CFL asked for more sub-steps than max_sub_steps_cap")
         if s & _lib.STATUS_SYNC_TIMEOUT:
-            raise RuntimeError("a grid barrier of the persistent interval kernel timed out")
+            raise RuntimeError("a wait of the interval kernel gave up; the state is undefined")
 
     # ------------------------------------------------------------------ #
     # ordering helpers, state I/O

@@ -673,8 +673,10 @@ int plan_resident(CmfPlan* p, const Layout& L)
 }
 
 // One interval through the resident kernel: the prologue, then the whole
-// interval in one cooperative launch.
-int interval_resident(CmfPlan* p, cudaStream_t s, double T, int fixed_n)
+// interval in one cooperative launch.  A test gives the polls of a wait and the
+// sub-step at which the last tile leaves.
+int interval_resident(CmfPlan* p, cudaStream_t s, double T, int fixed_n, unsigned polls = kWaitPolls,
+                      int leave_step = -1)
 {
     int rc;
     {
@@ -684,6 +686,8 @@ int interval_resident(CmfPlan* p, cudaStream_t s, double T, int fixed_n)
     }
     ResidentArgs ra = p->resident;
     ra.fixed_n = fixed_n;
+    ra.polls = polls;
+    ra.leave_step = leave_step;
     void* args[] = {p->dev, &p->stats, &ra};
     return check_cuda(cudaLaunchCooperativeKernel(p->ks.resident, dim3(p->resident_tiles),
                                                    dim3(p->resident_threads), args, p->resident.bytes, s));
@@ -1070,6 +1074,16 @@ int cmf_plan_set_persistent(CmfPlan* p, int enable)
 int cmf_plan_resident_tiles(const CmfPlan* p)
 {
     return p && p->graph_enabled && !p->persistent ? p->resident_tiles : 0;
+}
+
+int cmf_probe_resident_timeout(CmfPlan* p, void* stream, double outer_seconds, int32_t sub_steps, int32_t leave_step,
+                               int32_t polls)
+{
+    if (!p || !(outer_seconds > 0) || sub_steps <= 0 || leave_step < 0 || leave_step >= sub_steps || polls <= 0 ||
+        (unsigned)polls > kWaitPolls)
+        return CMF_ERR_ARG;
+    if (cmf_plan_resident_tiles(p) < 2) return CMF_ERR_UNSUPPORTED;
+    return interval_resident(p, (cudaStream_t)stream, outer_seconds, sub_steps, (unsigned)polls, leave_step);
 }
 
 int cmf_probe_barrier_timeout(void* stream, int32_t* control, int32_t* status, int32_t timeout_us)

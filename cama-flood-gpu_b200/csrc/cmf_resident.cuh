@@ -30,8 +30,10 @@
 //
 // A phase needs other tiles' values of earlier phases only, so no wait depends
 // on a thread of its own warp, and all CTAs are co-resident (cooperative
-// launch), so every wait ends.  Each is still bounded in time, after which
-// CMF_STATUS_SYNC_TIMEOUT and the abort word are set and every CTA leaves.
+// launch), so every wait ends.  Each is still bounded, in polls and not in time:
+// a process that is swapped off a shared GPU loses time but makes no polls.
+// After them CMF_STATUS_SYNC_TIMEOUT and the abort word are set and every CTA
+// leaves.
 #pragma once
 
 #include "cmf_device.cuh"
@@ -74,6 +76,8 @@ struct ResidentArgs {
     int tile;          // cells per tile
     TileCounts most;
     int fixed_n;       // > 0: the sub-step count, otherwise the CFL decides
+    unsigned polls;    // polls after which a wait gives up
+    int leave_step;    // sub-step at which the last tile leaves, for the test of that (-1: none)
     int o_rows;        // 0: the floodplain rows stay in L2
     int o_path, o_ends, o_levee, o_dam, o_halo, o_int, o_slot, o_flag;
     int bytes;
@@ -193,12 +197,18 @@ __device__ __forceinline__ void store_word(unsigned long long* p, unsigned long 
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(x) : "memory");
 }
 
-// One turn of a wait that began at t0: true when it has to give up, because it
-// has run out of time or another one has.  `quit` tells the CTA.
-__device__ __forceinline__ bool wait_over(int* ctl, int* status, unsigned long long t0, int* quit)
+// Polls of a wait, each an L2 round trip (some 0.3-0.7 us): seconds of a wait
+// that takes microseconds.
+constexpr unsigned kWaitPolls = 1u << 22;
+constexpr unsigned kPollsPerCheck = 64;  // between two looks at the abort word
+
+// A wait's look at how it stands after `spin` polls of at most `polls`: true
+// when it has to give up, because it has used them or another one has.  `quit`
+// tells the CTA.
+__device__ __forceinline__ bool wait_over(int* ctl, int* status, unsigned spin, unsigned polls, int* quit)
 {
     if (!*reinterpret_cast<volatile int*>(ctl + kCtlAbort)) {
-        if (global_ns() - t0 <= kBarrierTimeoutNs) return false;
+        if (spin < polls) return false;
         atomicOr(status, CMF_STATUS_SYNC_TIMEOUT);
         atomicExch(ctl + kCtlAbort, 1);
     }
@@ -213,15 +223,15 @@ __device__ __forceinline__ bool cta_quits(const int* quit)
 }
 
 // All tiles meet (once per interval, for the sub-step count); true: leave.
-__device__ __forceinline__ bool tiles_meet(unsigned* flags, int* ctl, int* status, int tiles, int* quit)
+__device__ __forceinline__ bool tiles_meet(unsigned* flags, int* ctl, int* status, int tiles, unsigned polls,
+                                           int* quit)
 {
     __syncthreads();
     if (threadIdx.x < 32) {
         if (threadIdx.x == 0) store_release_u32(flags + blockIdx.x, 1u);
         for (int q = threadIdx.x; q < tiles; q += 32) {
-            const unsigned long long t0 = global_ns();
-            while (load_acquire_u32(flags + q) == 0)
-                if (wait_over(ctl, status, t0, quit)) break;
+            for (unsigned spin = 1; load_acquire_u32(flags + q) == 0; ++spin)
+                if (spin % kPollsPerCheck == 0 && wait_over(ctl, status, spin, polls, quit)) break;
         }
     }
     return cta_quits(quit);
@@ -230,18 +240,17 @@ __device__ __forceinline__ bool tiles_meet(unsigned* flags, int* ctl, int* statu
 // What a CTA needs to wait for a word.
 struct Wait {
     int *ctl, *status, *quit;
-    unsigned epoch;
+    unsigned epoch, polls;
 };
 
 // The value bits of a word whose first read gave x, once it carries the epoch.
 __device__ __forceinline__ unsigned await_word(const unsigned long long* p, unsigned long long x, const Wait& w)
 {
     if ((unsigned)(x >> 32) != w.epoch) {
-        const unsigned long long t0 = global_ns();
         for (unsigned spin = 1;; ++spin) {
             x = load_word(p);
             if ((unsigned)(x >> 32) == w.epoch) break;
-            if (spin % 64 == 0 && wait_over(w.ctl, w.status, t0, w.quit)) break;
+            if (spin % kPollsPerCheck == 0 && wait_over(w.ctl, w.status, spin, w.polls, w.quit)) break;
         }
     }
     return (unsigned)x;
@@ -764,7 +773,7 @@ k_resident(const Dev<REAL> v, const StatsArgs stats, const ResidentArgs a)
     __shared__ int quit, step_max, own_paths, own_dams, levee_range[2], halo_lo, halo_hi, taken[2];
     const Tile<REAL> t = tile_of(v, a, smem);
     const int tid = threadIdx.x, nthr = blockDim.x;
-    Wait w{v.ctl, v.status, &quit, (unsigned)v.ctl[kCtlEpoch]};
+    Wait w{v.ctl, v.status, &quit, (unsigned)v.ctl[kCtlEpoch], a.polls};
 
     // ---- load the tile ----
     if (tid == 0) {
@@ -892,7 +901,7 @@ k_resident(const Dev<REAL> v, const StatsArgs stats, const ResidentArgs a)
         __syncthreads();
         if (tid == 0) atomicMax(&v.ctl[kCtlCflMax], step_max);
     }
-    if (tiles_meet(v.rflag, v.ctl, v.status, (int)gridDim.x, &quit)) return;
+    if (tiles_meet(v.rflag, v.ctl, v.status, (int)gridDim.x, a.polls, &quit)) return;
     if (n <= 0) n = __ldcg(v.ctl + kCtlCflMax);
     if (n < 1) n = 1;
     const int cap = v.max_sub_cap > 0 ? v.max_sub_cap : kHardSubStepCap;
@@ -920,6 +929,7 @@ k_resident(const Dev<REAL> v, const StatsArgs stats, const ResidentArgs a)
         return warps + __shfl_sync(0xffffffffu, c, 0);
     };
     for (int k = 0; k < n; ++k, ++w.epoch) {
+        if (k == a.leave_step && blockIdx.x == gridDim.x - 1) return;
         const bool diag = k == n - 1;
         const bool want_fraction = diag || stats.count > 0;
         for (int c = warps - 1 - warp; c < chunks; c = next_chunk(&taken[0])) {

@@ -44,7 +44,7 @@ extern "C" {
 /* ---- device status word bits (CmfView.status[0]) ------------------------- */
 #define CMF_STATUS_NONFINITE 1   /* NaN/Inf storage or discharge produced     */
 #define CMF_STATUS_SUBSTEP_CAP 2 /* CFL asked for more sub-steps than allowed */
-#define CMF_STATUS_SYNC_TIMEOUT 8 /* a grid barrier of the persistent interval kernel gave up */
+#define CMF_STATUS_SYNC_TIMEOUT 8 /* a wait of the resident or the persistent interval kernel gave up */
 
 /* ---- feature bits (CmfView.features) ------------------------------------- */
 #define CMF_FEAT_BIFURCATION 1 /* bifurcation module open                    */
@@ -236,14 +236,28 @@ void cmf_plan_destroy(CmfPlan* plan);
  * (CMF_ERR_UNSUPPORTED otherwise, and cmf_stats_attach refuses while it is
  * on); the grid is the device's resident CTAs, or fewer when the network
  * needs fewer.  A barrier wait that outlasts 1 s raises
- * CMF_STATUS_SYNC_TIMEOUT and ends the interval.  enable == 0 returns to the
+ * CMF_STATUS_SYNC_TIMEOUT and ends the interval; the state is then undefined.  enable == 0 returns to the
  * interval graph. */
 int cmf_plan_set_persistent(CmfPlan* plan, int enable);
 /* Tiles of the resident interval kernel that cmf_step_interval takes for this
  * plan: one member without budget whose state fits the SMs' shared memory runs
  * a whole interval in one cooperative launch after the prologue (the interval
- * graph inside a stream capture).  0: the plan takes another form. */
+ * graph inside a stream capture).  0: the plan takes another form.  Its blocks
+ * wait for one another's values; a wait that has polled 2^22 times without
+ * success (seconds, where microseconds are usual) raises
+ * CMF_STATUS_SYNC_TIMEOUT and ends the interval, and the state and the
+ * statistics are then undefined: blocks that need nothing of the one that
+ * failed may have written theirs. */
 int cmf_plan_resident_tiles(const CmfPlan* plan);
+/* Test of the resident kernel's failure path (no counterpart in the
+ * reference): runs an interval of `sub_steps` through the resident kernel
+ * whose last tile leaves at sub-step leave_step (0 .. sub_steps - 1), so the
+ * tiles that exchange values with it wait for words that nothing posts.  Each
+ * wait gives up after `polls` (1 .. 2^22) polls, sets CMF_STATUS_SYNC_TIMEOUT,
+ * and every block returns; nothing hangs.  CMF_ERR_UNSUPPORTED for a plan of
+ * fewer than two resident tiles. */
+int cmf_probe_resident_timeout(CmfPlan* plan, void* stream, double outer_seconds, int32_t sub_steps,
+                               int32_t leave_step, int32_t polls);
 
 /* Test of the persistent kernel's failure path (no counterpart in the
  * reference): launches, cooperatively, two blocks that meet at a grid barrier
