@@ -92,7 +92,7 @@ constexpr int kCtlMaxSteps = 1;   // max over members of the sub-step count
 constexpr int kCtlBarrier = 4;    // [4..5]: arrival counter (u64) of the persistent kernel's grid barrier
 constexpr int kCtlAbort = 6;      // set when a grid barrier gave up: every block leaves the interval
 constexpr int kCtlCflMax = 8;     // resident kernel: CFL sub-step count, maximum over the tiles
-constexpr int kCtlEpoch = 9;      // resident kernel: last epoch of the exchanged values
+constexpr int kCtlEpoch = 9;      // resident kernel: last epoch that exchanged values may carry
 constexpr int kCtlTileMax = 10;   // [10..15]: TileScan of the resident kernel
 constexpr int kResidentMaxTiles = 256;  // flags of the resident kernel (cmf_resident.cuh)
 constexpr int kHardSubStepCap = 100000;  // bound of the device-side sub-step loop

@@ -910,6 +910,10 @@ k_resident(const Dev<REAL> v, const StatsArgs stats, const ResidentArgs a)
         n = cap;
     }
     const REAL dt = (REAL)(v.tsec[0] / (double)n);
+    // The epochs of this interval are taken from here on, by every tile that gets
+    // here: all have read the last one, and an interval that is given up leaves
+    // words with them, which the next one must not take for its own.
+    if (tid == 0) v.ctl[kCtlEpoch] = (int)(w.epoch + 1 + n);
     w.epoch += 1;
     for (int j = tid; j < t.count; j += nthr) publish_state<REAL, RES, LEV, BIF>(v, t, j, w.epoch);
 
@@ -1018,7 +1022,6 @@ k_resident(const Dev<REAL> v, const StatsArgs stats, const ResidentArgs a)
         v.cur[0] = n - 1;
         v.ctl[kCtlMaxSteps] = n;
         v.ctl[kCtlStep] = n;
-        v.ctl[kCtlEpoch] = (int)w.epoch;
     }
 }
 

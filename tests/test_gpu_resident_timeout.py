@@ -1,7 +1,8 @@
 """The waits of the resident interval kernel are bounded: a tile that leaves in
 the middle of an interval (and posts nothing more) makes those that need its
 values give up after their polls, report it in the status word and leave; the
-kernel returns and the context stays usable."""
+kernel returns, the context stays usable, and the plan runs on from a restored
+state."""
 import time
 
 import numpy as np
@@ -48,6 +49,28 @@ def test_resident_wait_gives_up_and_reports(case, precision, leave, device):
     _give_up(m, leave)
     x = torch.arange(100, device=device, dtype=torch.float32)
     assert float(x.sum().item()) == 4950.0
+
+
+@pytest.mark.parametrize("case, precision", [("plain", "float32"), ("full", "float32"), ("full", "float64")])
+def test_resident_plan_runs_on_after_a_give_up(case, precision, device):
+    """The words that the abandoned interval left are not taken for the next
+    one's: with the state restored, the plan equals one that never failed."""
+    net, m = _model(case, precision)
+    ref = _model(case, precision)[1]
+    before = {k: v.clone() for k, v in m.state_tensors().items()}
+    for leave in (0, 1, SUB_STEPS - 1):
+        _give_up(m, leave)
+        for k, v in m.state_tensors().items():
+            v.copy_(before[k])
+        m._status.zero_()
+    for d in range(2):
+        for x in (m, ref):
+            x.set_inputs(torch.as_tensor(x.to_model_order(20.0 * syn.daily_runoff(net, d))).cuda())
+            x.step_advance()
+    torch.cuda.synchronize()
+    m.check_status()
+    for k, v in ref.state_tensors().items():
+        np.testing.assert_array_equal(m.state_tensors()[k].cpu().numpy(), v.cpu().numpy(), err_msg=k)
 
 
 def test_resident_probe_refuses_what_it_does_not_run(device):
