@@ -172,6 +172,8 @@ def lib() -> ctypes.CDLL:
     h.cmf_plan_set_member_tile.argtypes = [_P, _I32]
     h.cmf_plan_resident_tiles.restype = ctypes.c_int
     h.cmf_plan_resident_tiles.argtypes = [_P]
+    h.cmf_plan_set_resident.restype = ctypes.c_int
+    h.cmf_plan_set_resident.argtypes = [_P, ctypes.c_int]
     h.cmf_probe_resident_timeout.restype = ctypes.c_int
     h.cmf_probe_resident_timeout.argtypes = [_P, _P, _F64, _I32, _I32, _I32]
     h.cmf_plan_set_persistent.restype = ctypes.c_int

@@ -138,7 +138,8 @@ class CaMaFlood:
     "last": ["river_depth"]}, scripts/run_daily_bin.py:28) and accumulates
     those statistics on the device after every sub-step; `collect_statistics()`
     ends an output period (no file writer: the reference's NetCDF output
-    workers are outside this path).
+    workers are outside this path).  `persistent` and `resident` choose the
+    form of an interval (set_persistent, set_resident).
     """
 
     def __init__(self, device: str | torch.device = "cuda", input_proxy: Optional[Mapping] = None,
@@ -150,7 +151,7 @@ class CaMaFlood:
                  gravity: float = 9.8, min_kinematic_slope: float = 1.0e-5,
                  adaptive_time_factor: float = 0.7, budget: bool = False,
                  variables_to_save: Optional[Mapping[str, Iterable[str]]] = None,
-                 persistent: bool = False):
+                 persistent: bool = False, resident: bool = True):
         if input_proxy is None:
             raise ValueError("input_proxy (field name -> array mapping) is required")
         mods = set(opened_modules) | {"base"}
@@ -179,6 +180,7 @@ class CaMaFlood:
         self.budget_enabled = bool(budget) or "log" in mods
         self.member_tile = 1
         self.persistent = False
+        self.resident = bool(resident)
         self._plan = None
         self._prepare(dict(input_proxy), dict(batched_fields or {}))
         self._upload()
@@ -568,6 +570,8 @@ class CaMaFlood:
         self._attach_statistics()
         if self.persistent:
             _lib.check(lib.cmf_plan_set_persistent(plan, 1), "plan_set_persistent")
+        if not self.resident:
+            _lib.check(lib.cmf_plan_set_resident(plan, 0), "plan_set_resident")
 
     # ------------------------------------------------------------------ #
     # output statistics (variables_to_save)
@@ -805,6 +809,13 @@ class CaMaFlood:
                              "output statistics")
         _lib.check(rc, "plan_set_persistent")
         self.persistent = bool(on)
+
+    def set_resident(self, on: bool = True) -> None:
+        """Whether a network that fits the SMs' shared memory runs its
+        intervals in the resident kernel (the default) or through the interval
+        graph; the results are the same."""
+        _lib.check(_lib.lib().cmf_plan_set_resident(self._plan, 1 if on else 0), "plan_set_resident")
+        self.resident = bool(on)
 
     @property
     def resident_tiles(self) -> int:

@@ -203,7 +203,9 @@ struct CmfPlan {
     // persistent interval kernel instead of the interval graph
     bool persistent;
     int persist_grid;
-    // resident interval kernel: its tiles (0: the network does not fit)
+    // resident interval kernel: its tiles (0: the network does not fit), and
+    // whether the caller has turned it off
+    bool resident_off;
     ResidentArgs resident;
     int resident_tiles;
     int resident_threads;
@@ -880,7 +882,7 @@ int cmf_step_interval(CmfPlan* p, void* stream, double outer_seconds, int32_t fi
     if (p->persistent) return interval_persistent(p, s, outer_seconds, fixed);
     if (!p->graph_enabled) return interval_direct(p, s, outer_seconds, fixed);
     int rc;
-    if (p->resident_tiles > 0) {
+    if (cmf_plan_resident_tiles(p) > 0) {
         // a stream capture takes the interval graph, as it always has
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone)
@@ -1071,9 +1073,16 @@ int cmf_plan_set_persistent(CmfPlan* p, int enable)
     return CMF_OK;
 }
 
+int cmf_plan_set_resident(CmfPlan* p, int enable)
+{
+    if (!p) return CMF_ERR_ARG;
+    p->resident_off = !enable;
+    return CMF_OK;
+}
+
 int cmf_plan_resident_tiles(const CmfPlan* p)
 {
-    return p && p->graph_enabled && !p->persistent ? p->resident_tiles : 0;
+    return p && p->graph_enabled && !p->persistent && !p->resident_off ? p->resident_tiles : 0;
 }
 
 int cmf_probe_resident_timeout(CmfPlan* p, void* stream, double outer_seconds, int32_t sub_steps, int32_t leave_step,

@@ -249,6 +249,10 @@ int cmf_plan_set_persistent(CmfPlan* plan, int enable);
  * statistics are then undefined: blocks that need nothing of the one that
  * failed may have written theirs. */
 int cmf_plan_resident_tiles(const CmfPlan* plan);
+/* enable == 0: such a plan runs its intervals through the interval graph
+ * instead, with the same results; enable != 0 (the default) returns to the
+ * resident kernel. */
+int cmf_plan_set_resident(CmfPlan* plan, int enable);
 /* Test of the resident kernel's failure path (no counterpart in the
  * reference): runs an interval of `sub_steps` through the resident kernel
  * whose last tile leaves at sub-step leave_step (0 .. sub_steps - 1), so the
