@@ -882,12 +882,12 @@ int cmf_step_interval(CmfPlan* p, void* stream, double outer_seconds, int32_t fi
     if (p->persistent) return interval_persistent(p, s, outer_seconds, fixed);
     if (!p->graph_enabled) return interval_direct(p, s, outer_seconds, fixed);
     int rc;
-    if (cmf_plan_resident_tiles(p) > 0) {
-        // a stream capture takes the interval graph, as it always has
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone)
-            return interval_resident(p, s, outer_seconds, fixed);
-    }
+    // The interval graph has a conditional node, which a child graph may not
+    // hold: CUDA refuses it inside a stream capture and spoils the capture.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if ((rc = check_cuda(cudaStreamIsCapturing(s, &capture))) != CMF_OK) return rc;
+    if (capture != cudaStreamCaptureStatusNone) return CMF_ERR_UNSUPPORTED;
+    if (cmf_plan_resident_tiles(p) > 0) return interval_resident(p, s, outer_seconds, fixed);
     const bool adaptive_now = fixed == 0;
     if (p->graph_ready) {
         const bool was_adaptive = p->graph_fixed == 0;

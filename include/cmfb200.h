@@ -241,8 +241,7 @@ void cmf_plan_destroy(CmfPlan* plan);
 int cmf_plan_set_persistent(CmfPlan* plan, int enable);
 /* Tiles of the resident interval kernel that cmf_step_interval takes for this
  * plan: one member without budget whose state fits the SMs' shared memory runs
- * a whole interval in one cooperative launch after the prologue (the interval
- * graph inside a stream capture).  0: the plan takes another form.  Its blocks
+ * a whole interval in one cooperative launch after the prologue.  0: the plan takes another form.  Its blocks
  * wait for one another's values; a wait that has polled 2^22 times without
  * success (seconds, where microseconds are usual) raises
  * CMF_STATUS_SYNC_TIMEOUT and ends the interval, and the state and the
@@ -283,7 +282,10 @@ int cmf_plan_set_member_tile(CmfPlan* plan, int32_t width);
  * CaMaFlood.step_advance (cmfgpu/models/cama_flood_model.py:104-173):
  * adaptive sub-step count on the device (no host sync), dt = T / n, then n
  * sub-steps of momentum -> limiter/inflow/stage.  fixed_sub_steps > 0 skips
- * the CFL and uses that count (the reference's fixed mode). */
+ * the CFL and uses that count (the reference's fixed mode).  Inside a stream
+ * capture a plan with CMF_FEAT_GRAPH returns CMF_ERR_UNSUPPORTED and leaves the
+ * capture as it is: the interval graph has a conditional node, which CUDA does
+ * not take into a captured graph (cmf_substep_noalloc can be captured). */
 int cmf_step_interval(CmfPlan* plan, void* stream, double outer_seconds,
                       int32_t fixed_sub_steps);
 
