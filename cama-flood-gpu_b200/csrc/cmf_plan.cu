@@ -668,6 +668,11 @@ int plan_resident(CmfPlan* p, const Layout& L)
     const int most = p->fp64 ? resident_threads<double>() : resident_threads<float>();
     const int threads = tile + 32 * ceil_div(a.most.paths, 32 / kPathLanes);
     p->resident_threads = threads < most ? threads : most;
+    int per_sm = 0;
+    if ((rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p->ks.resident, p->resident_threads,
+                                                                       a.bytes))) != CMF_OK)
+        return rc;
+    if (per_sm * sms < tiles) return CMF_OK;  // not co-resident
     // no word may carry an epoch that this plan will use
     if ((rc = check_cuda(cudaMemset(ws + L.rflag, 0, L.x_end - L.rflag))) != CMF_OK) return rc;
     p->resident_tiles = tiles;
@@ -691,8 +696,11 @@ int interval_resident(CmfPlan* p, cudaStream_t s, double T, int fixed_n, unsigne
     ra.polls = polls;
     ra.leave_step = leave_step;
     void* args[] = {p->dev, &p->stats, &ra};
-    return check_cuda(cudaLaunchCooperativeKernel(p->ks.resident, dim3(p->resident_tiles),
-                                                   dim3(p->resident_threads), args, p->resident.bytes, s));
+    const cudaError_t e = cudaLaunchCooperativeKernel(p->ks.resident, dim3(p->resident_tiles),
+                                                      dim3(p->resident_threads), args, p->resident.bytes, s);
+    if (e != cudaErrorCooperativeLaunchTooLarge) return check_cuda(e);
+    (void)cudaGetLastError();
+    return CMF_ERR_UNSUPPORTED;
 }
 
 // One interval through the persistent kernel: the prologue kernels, then
@@ -887,7 +895,11 @@ int cmf_step_interval(CmfPlan* p, void* stream, double outer_seconds, int32_t fi
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if ((rc = check_cuda(cudaStreamIsCapturing(s, &capture))) != CMF_OK) return rc;
     if (capture != cudaStreamCaptureStatusNone) return CMF_ERR_UNSUPPORTED;
-    if (cmf_plan_resident_tiles(p) > 0) return interval_resident(p, s, outer_seconds, fixed);
+    if (cmf_plan_resident_tiles(p) > 0) {
+        rc = interval_resident(p, s, outer_seconds, fixed);
+        if (rc != CMF_ERR_UNSUPPORTED) return rc;
+        p->resident_tiles = 0;  // the tiles no longer fit the device together
+    }
     const bool adaptive_now = fixed == 0;
     if (p->graph_ready) {
         const bool was_adaptive = p->graph_fixed == 0;
