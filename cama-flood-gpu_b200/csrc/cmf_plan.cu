@@ -34,6 +34,19 @@ constexpr int kDefaultBlock = 256;
 // catchments: 14.0, 13.3, 12.1, 14.1 and 14.5 us per sub-step at 32, 64, 128,
 // 256 and 512 cells).
 constexpr int kResidentMinTile = 128;
+// Most path ends of a cell and of a tile that the resident kernel takes.  One
+// thread loads a cell's ends, folds them in order and publishes the cell's state
+// and rate to each path elsewhere.  With one cell of h ends, through the interval
+// graph and through this kernel, a single sub-step and an hour (25-28 sub-steps):
+// 60k catchments 53 / 44 us and 0.89 / 0.50 ms at h = 32, 57 / 60 us and 1.02 /
+// 0.70 ms at 64, 94 / 152 us and 1.97 / 1.97 ms at 256, 227 / 527 us and 5.5 / 6.9
+// ms at 1,024; 4k catchments 55 / 40 us and 1.05 / 0.53 ms at 32, 59 / 56 us and
+// 1.22 / 0.75 ms at 64, 133 / 273 us and 3.2 / 3.8 ms at 512.  A tile's ends cost
+// it an exchange each: paths between random cells, 830 ends per tile (60k
+// catchments and paths) 55 / 56 us and 1.04 / 0.82 ms, 1,410 (100k and 100k) 61 /
+// 73 us and 1.25 / 1.16 ms.
+constexpr int kResidentCellEnds = 48;
+constexpr int kResidentTileEnds = 1024;
 
 struct KernelSet {
     const void* momentum;
@@ -140,7 +153,7 @@ Layout layout_of(const CmfView* v, int cell_blocks)
     L.rs1 = o; o = align_up(o + nm * 8);
     L.fs1 = o; o = align_up(o + nm * 8);
     L.bpart = o; o = align_up(o + (size_t)kBudgetTerms * (size_t)cell_blocks * 8);
-    L.ctl = o; o = align_up(o + 16 * sizeof(int));
+    L.ctl = o; o = align_up(o + kCtlWords * sizeof(int));
     L.tsec = o; o = align_up(o + 8);
     L.base_total = o;
     const size_t nlv = (v->features & CMF_FEAT_LEVEE) ? (size_t)v->num_levees : 0;
@@ -651,11 +664,11 @@ int plan_resident(CmfPlan* p, const Layout& L)
     const void* scan = p->fp64 ? (const void*)k_resident_scan<double> : (const void*)k_resident_scan<float>;
     if ((rc = launch(scan, tiles, 256, args, 0)) != CMF_OK) return rc;
     TileScan found;
-    static_assert(kCtlTileMax + sizeof(TileScan) / sizeof(int) <= 16, "the control words end here");
+    static_assert(kCtlTileMax + sizeof(TileScan) / sizeof(int) <= kCtlWords, "the control words end here");
     if ((rc = check_cuda(cudaMemcpy(&found, (int*)(ws + L.ctl) + kCtlTileMax, sizeof(found),
                                     cudaMemcpyDeviceToHost))) != CMF_OK)
         return rc;
-    if (found.irregular) return CMF_OK;
+    if (found.irregular || found.cell_ends > kResidentCellEnds || found.most.ends > kResidentTileEnds) return CMF_OK;
     a.most = found.most;
     resident_layout(a, real, v.num_flood_levels, v.num_bifurcation_levels, true);
     if (a.bytes > room) resident_layout(a, real, v.num_flood_levels, v.num_bifurcation_levels, false);

@@ -719,20 +719,22 @@ __device__ __forceinline__ int first_at_least(const int* list, int n, int x)
 struct TileScan {
     TileCounts most;  // maxima over the tiles
     int irregular;    // not 0: the view's lists are not in the form below
+    int cell_ends;    // the most path ends of a cell
 };
 
 // TileCounts of every tile (one block each) and the form of the lists that
 // k_resident indexes by, once per plan.  A levee of the tile is found by
 // bisection of the levee list and writes its cell's slot, so the list has to be
 // strictly ascending, in range, and exactly the cells flagged as levee cells;
-// a path end elsewhere answers only if its cell is flagged for bifurcation.
+// a path end elsewhere answers only if its cell is flagged for bifurcation and
+// is the one that the path names.
 // The sub-step kernels ask for neither (levee_slot maps any order).
 template <typename REAL>
 __global__ void __launch_bounds__(256) k_resident_scan(const Dev<REAL> v, int tile)
 {
-    __shared__ int own, dams, levees, bad, lo, hi;
+    __shared__ int own, dams, levees, bad, lo, hi, cell_ends;
     const int t0 = blockIdx.x * tile, t1 = min(t0 + tile, (int)v.N);
-    if (threadIdx.x == 0) { own = dams = levees = bad = hi = 0; lo = INT32_MAX; }
+    if (threadIdx.x == 0) { own = dams = levees = bad = hi = cell_ends = 0; lo = INT32_MAX; }
     __syncthreads();
     for (int i = t0 + threadIdx.x; i < t1; i += blockDim.x) {
         const int c0 = v.up[i], c1 = upstream_end(v, (long)i);
@@ -743,11 +745,19 @@ __global__ void __launch_bounds__(256) k_resident_scan(const Dev<REAL> v, int ti
         }
         if ((v.features & CMF_FEAT_RESERVOIR) && (fl & CMF_CELL_RESERVOIR)) atomicAdd(&dams, 1);
         if ((v.features & CMF_FEAT_LEVEE) && (fl & CMF_CELL_LEVEE)) atomicAdd(&levees, 1);
-        if ((v.features & CMF_FEAT_BIFURCATION) && v.bptr[i] < v.bptr[i + 1] && !(fl & CMF_CELL_BIFURCATION)) bad = 1;
+        if ((v.features & CMF_FEAT_BIFURCATION) && v.bptr[i] < v.bptr[i + 1]) {
+            if (!(fl & CMF_CELL_BIFURCATION)) bad = 1;
+            atomicMax(&cell_ends, v.bptr[i + 1] - v.bptr[i]);
+        }
     }
     if (v.features & CMF_FEAT_BIFURCATION)
-        for (int x = v.bptr[t0] + threadIdx.x; x < v.bptr[t1]; x += blockDim.x)
-            if (!(v.bpaths[x] & 1)) atomicAdd(&own, 1);
+        for (int x = v.bptr[t0] + threadIdx.x; x < v.bptr[t1]; x += blockDim.x) {
+            const int e = v.bpaths[x];
+            if (!(e & 1)) atomicAdd(&own, 1);
+            const bool path = e >= 0 && (e >> 1) < v.P;
+            const int c = !path ? -1 : (e & 1) ? v.bdi[e >> 1] : v.bci[e >> 1];
+            if (c < t0 || c >= t1 || x < v.bptr[c] || x >= v.bptr[c + 1]) bad = 1;
+        }
     for (long l = (long)blockIdx.x * blockDim.x + threadIdx.x; l < v.NLV; l += (long)gridDim.x * blockDim.x) {
         const int c = v.lci[l];
         if (c < 0 || c >= v.N || (l > 0 && v.lci[l - 1] >= c) || !(v.flags[c] & CMF_CELL_LEVEE)) bad = 1;
@@ -763,6 +773,7 @@ __global__ void __launch_bounds__(256) k_resident_scan(const Dev<REAL> v, int ti
     atomicMax(most + 3, dams);
     if (hi > 0) atomicMax(most + 4, hi - lo);
     if (bad || levees != listed) atomicMax(most + 5, 1);
+    atomicMax(most + 6, cell_ends);
 }
 
 template <typename REAL, bool RES, bool LEV, bool BIF>

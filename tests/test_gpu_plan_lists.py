@@ -2,8 +2,9 @@
 a levee list that is not ascending, a levee cell that no levee lists, a path end
 in a cell that is not flagged for bifurcation.  The plan leaves such a view to
 the interval graph, whose results are those of the same view with the sub-step
-kernels launched one by one.  Flag bits that the library does not define change
-nothing."""
+kernels launched one by one; it does the same where a cell or a tile has more
+path ends than the resident kernel is fast with.  Flag bits that the library does
+not define change nothing."""
 import numpy as np
 import pytest
 import torch
@@ -82,3 +83,46 @@ def test_undefined_flag_bits_are_ignored(device):
     marked._rebuild_plan(marked.block_size)
     assert marked.resident_tiles > 0
     _same(_run(plain, net), _run(marked, net))
+
+
+def _paths(n, count, hub_ends, seed=5):
+    """`count` paths between random cells, `hub_ends` of them into the last cell."""
+    net = syn.generate(syn.NetworkSpec(n, seed=1, bifurcation_paths=count, levee_fraction=0.2))
+    rng = np.random.default_rng(seed)
+    net.fields["bifurcation_catchment_id"] = rng.integers(0, n - 1, size=count)
+    to = rng.integers(0, n - 1, size=count)
+    to[:hub_ends] = n - 1
+    net.fields["bifurcation_downstream_id"] = to
+    return net
+
+
+@pytest.mark.parametrize("precision", ["float32", "float64"])
+@pytest.mark.parametrize("n, count, hub_ends, resident", [
+    (6000, 400, 48, True), (6000, 400, 49, False),         # the most path ends of a cell
+    (2500, 8000, 0, True), (2500, 12_000, 0, False)])      # 819 and 1,229 in a tile
+def test_cells_and_tiles_with_many_path_ends(n, count, hub_ends, resident, precision, device):
+    net = _paths(n, count, hub_ends)
+    runs = []
+    for graph in (True, False):
+        m = P.model_for(net, precision=precision, use_cuda_graph=graph)
+        assert (m.resident_tiles > 0) == (graph and resident)
+        runs.append(_run(m, net, days=1))
+    _same(*runs)
+
+
+def test_path_in_the_wrong_cells_list(device):
+    """Two cells' lists exchanged: the resident kernel takes one end's cell from the list
+    and the other's from the path."""
+    net = P.make_network("bif", n=5000)
+    runs = []
+    for graph in (True, False):
+        m = P.model_for(net, use_cuda_graph=graph)
+        b = m.bifurcation
+        n_ends = (b.bif_cell_ptr[1:] - b.bif_cell_ptr[:-1]).cpu().numpy()
+        i, j = np.flatnonzero(n_ends == 1)[[3, 40]]
+        x, y = int(b.bif_cell_ptr[i]), int(b.bif_cell_ptr[j])
+        b.bif_cell_paths[[x, y]] = b.bif_cell_paths[[y, x]]
+        m._rebuild_plan(m.block_size)
+        assert m.resident_tiles == 0
+        runs.append(_run(m, net, days=1))
+    _same(*runs)
