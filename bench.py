@@ -506,11 +506,12 @@ def small_network_measure(device, name: str, days: int) -> dict:
     """One of the small benchmark configurations (plain_60k: 60,000
     catchments, plain physics, daily runoff, the 3600 s dt cap; full_250k:
     250,000 catchments with full physics) routed through the public API over
-    `days` daily intervals after one warm-up day, three ways on the same GPU:
-    the interval graph, the persistent interval kernel, and the reference's
-    own CUDA kernels (oracle/_ref, driven as CaMaFlood.step_advance drives
-    them).  A sub-step here is a few microseconds of work, so launch and
-    barrier costs decide.  The three end states are compared field by field.
+    `days` daily intervals after one warm-up day, four ways on the same GPU:
+    the resident kernel (what a model of this size runs by default), the
+    interval graph, the persistent interval kernel, and the reference's own
+    CUDA kernels (oracle/_ref, driven as CaMaFlood.step_advance drives them).
+    A sub-step here is a few microseconds of work, so launch, barrier and
+    exchange costs decide.  The end states are compared field by field.
     The reference has no dt cap, so on plain_60k its arm runs the capped count
     max(n, T / 3600 s) as a fixed count, as the parity test does."""
     import torch
@@ -524,9 +525,12 @@ def small_network_measure(device, name: str, days: int) -> dict:
     out = {"catchments": net.num_catchments, "days": days, "warmup_days": 1,
            "modules": list(net.opened_modules)}
     states = {}
-    for mode in ("graph", "persistent"):
+    for mode in ("resident", "graph", "persistent"):
         m = CaMaFlood(device=device, input_proxy=net.fields, opened_modules=net.opened_modules,
-                      step_duration=T, max_sub_step_seconds=cap_s, persistent=(mode == "persistent"))
+                      step_duration=T, max_sub_step_seconds=cap_s, persistent=(mode == "persistent"),
+                      resident=(mode == "resident"))
+        if (m.resident_tiles > 0) != (mode == "resident"):
+            raise RuntimeError(f"{name} does not run in the {mode} form")
         run = [torch.as_tensor(syn.daily_runoff(net, d)[m.order]).to(device) for d in range(days + 1)]
         m.set_inputs(run[0])
         m.step_advance()
@@ -548,9 +552,10 @@ def small_network_measure(device, name: str, days: int) -> dict:
         states[mode] = {k: v.cpu().numpy().copy() for k, v in m.state_tensors().items()}
         order = m.order
         m.close()
-    out["persistent_over_graph"] = out["persistent"]["value"] / out["graph"]["value"]
-    out["persistent_state_equal"] = all(np.array_equal(states["graph"][k], states["persistent"][k])
-                                        for k in states["graph"])
+    for mode in ("resident", "persistent"):
+        out[f"{mode}_over_graph"] = out[mode]["value"] / out["graph"]["value"]
+        out[f"{mode}_state_equal"] = all(np.array_equal(states["graph"][k], states[mode][k])
+                                         for k in states["graph"])
     if RC.available():
         ref = RC.RefCuda(O.reference_fields(net.fields, net.opened_modules), net.opened_modules,
                          device=device)
@@ -583,7 +588,7 @@ def small_network_measure(device, name: str, days: int) -> dict:
                 b = b[order]
             equal = equal and bool(np.array_equal(a, b))
         out["reference_cuda"]["state_equal"] = equal
-        best = max(out["graph"]["value"], out["persistent"]["value"])
+        best = max(out[mode]["value"] for mode in states)
         out["ours_best_over_reference_cuda"] = best / out["reference_cuda"]["value"]
         del ref
     return out
@@ -1345,7 +1350,8 @@ def main() -> None:
                     help="skip timing the reference's own CUDA kernels on the same workload")
     ap.add_argument("--no-small-networks", dest="small_networks", action="store_false",
                     help="skip the small-configuration leg (60k plain and 250k full physics: "
-                         "interval graph, persistent kernel and the reference's CUDA kernels)")
+                         "resident kernel, interval graph, persistent kernel and the reference's "
+                         "CUDA kernels)")
     ap.add_argument("--probe-ensemble", action="store_true",
                     help="with --probe-kernels: probe the member-batched kernels of the ensemble "
                          "workload instead")
