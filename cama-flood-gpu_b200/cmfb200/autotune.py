@@ -63,9 +63,11 @@ def tune_block_size(model, candidates: Iterable[int] = DEFAULT_CANDIDATES, sub_s
                     tile_candidates: Optional[Iterable[int]] = None) -> dict:
     """Pick the fastest block size (and member tile) for `model`, leave the
     model's plan built with them and return {"block_size": b, "member_tile":
-    w, "ms_per_sub_step": {b: ms} (one member) or {"b/w": ms}, "cached": bool}.
-    Tile candidates default to the divisors of the member count in
-    DEFAULT_TILES (just 1 for one member).
+    w, "ms_per_sub_step": {b: ms} (one member) or {"b/w": ms}, "cached": bool,
+    "used_by_step_advance": bool}.  Tile candidates default to the divisors of
+    the member count in DEFAULT_TILES (just 1 for one member).  A network whose
+    intervals run in the resident kernel (model.resident_tiles > 0) uses the
+    choice in the per-phase entry points only: "used_by_step_advance" is False.
 
     The model's state after the call equals its state before the call."""
     M = model.num_members
@@ -85,7 +87,7 @@ def tune_block_size(model, candidates: Iterable[int] = DEFAULT_CANDIDATES, sub_s
         if w != model.member_tile:
             model.set_member_tile(w)
         return {"block_size": b, "member_tile": w, "ms_per_sub_step": cache[key]["ms_per_sub_step"],
-                "cached": True}
+                "cached": True, "used_by_step_advance": not getattr(model, "resident_tiles", 0)}
 
     snapshot = {k: v.clone() for k, v in model.state_tensors().items()}
     original = (model.block_size, model.member_tile)
@@ -119,4 +121,5 @@ def tune_block_size(model, candidates: Iterable[int] = DEFAULT_CANDIDATES, sub_s
                       "ms_per_sub_step": {str(k): v for k, v in shown.items()}}
         with open(cache_path, "w") as fh:
             json.dump(cache, fh, indent=1, sort_keys=True)
-    return {"block_size": best_b, "member_tile": best_w, "ms_per_sub_step": shown, "cached": False}
+    return {"block_size": best_b, "member_tile": best_w, "ms_per_sub_step": shown, "cached": False,
+            "used_by_step_advance": not getattr(model, "resident_tiles", 0)}

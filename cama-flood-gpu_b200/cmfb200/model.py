@@ -827,8 +827,10 @@ class CaMaFlood:
     def autotune_block_size(self, candidates=None, sub_steps: int = 6,
                             cache_path: Optional[str] = None, tile_candidates=None) -> dict:
         """Measure the candidate CTA sizes (and, with several members, member
-        tiles) on this network and keep the fastest
-        (cmfb200.autotune.tune_block_size); the state is unchanged."""
+        tiles) of the sub-step kernels on this network and keep the fastest
+        (cmfb200.autotune.tune_block_size); the state is unchanged.  The
+        resident kernel, which small networks run by themselves, does not
+        depend on the choice."""
         from .autotune import DEFAULT_CANDIDATES, tune_block_size
         return tune_block_size(self, candidates or DEFAULT_CANDIDATES, sub_steps,
                                cache_path=cache_path, tile_candidates=tile_candidates)
