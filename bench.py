@@ -660,7 +660,7 @@ def adjoint_compare(device, days: int, checkpoint_every: int = 96, repeats: int 
         ta.append(ev[2].elapsed_time(ev[3]) / 1e3)
     t_fwd = statistics.median(tf)
     t_adj = statistics.median(ta)
-    # the product's own fp64 forward (interval graphs) over the same window
+    # the product's own fp64 forward over the same window
     snap = {k: v.clone() for k, v in model.state_tensors().items()}
     b = model.base
     for k in ("river_manning", "flood_manning", "river_height", "river_width"):
@@ -712,6 +712,7 @@ def adjoint_compare(device, days: int, checkpoint_every: int = 96, repeats: int 
         torch.cuda.synchronize(device)
         tm.append(ev[0].elapsed_time(ev[1]) / 1e3)
     t_mixed = statistics.median(tm)
+    form = ["resident kernel" if m.resident_tiles else "interval graphs" for m in (model, mixed)]
     mixed.close()
     # sub-step count of the window (the CFL counts of the primal run)
     _, _, counts, _, _ = eng._forward(params["river_manning"], params["flood_manning"],
@@ -747,8 +748,9 @@ def adjoint_compare(device, days: int, checkpoint_every: int = 96, repeats: int 
             "workload": "full-physics 250k network, fp64, daily forcing, gradients w.r.t. "
                         "river Manning, river height, river width and runoff; fwd = the same "
                         "primal kernels without checkpoints; product_fwd = CaMaFlood.step_advance "
-                        "in fp64 (interval graphs) over the same window; mixed_product_fwd = the "
-                        "same in the reference's mixed precision (fp32 fluxes, fp64 storage)"}
+                        f"in fp64 ({form[0]}) over the same window; mixed_product_fwd = the "
+                        "same in the reference's mixed precision (fp32 fluxes, fp64 storage; "
+                        f"{form[1]})"}
 
 
 def adjoint_fd_check(device, days: int, cells: int, seed: int = 5) -> dict:

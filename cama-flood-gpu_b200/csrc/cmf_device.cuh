@@ -90,7 +90,7 @@ constexpr int kCtlStep = 0;    // index k that k_momentum reads
 constexpr int kCtlStepOf = 2;  // index k that the other kernels of the sub-step read
 constexpr int kCtlMaxSteps = 1;   // max over members of the sub-step count
 constexpr int kCtlBarrier = 4;    // [4..5]: arrival counter (u64) of the persistent kernel's grid barrier
-constexpr int kCtlAbort = 6;      // set when a grid barrier gave up: every block leaves the interval
+constexpr int kCtlAbort = 6;      // set when a wait gave up: every block leaves the interval
 constexpr int kCtlCflMax = 8;     // resident kernel: CFL sub-step count, maximum over the tiles
 constexpr int kCtlEpoch = 9;      // resident kernel: last epoch that exchanged values may carry
 constexpr int kCtlTileMax = 10;   // [10..16]: TileScan of the resident kernel

@@ -12,7 +12,8 @@
 //         -> [budget flush]
 //
 // so a whole forcing interval is one cudaGraphLaunch with the sub-step count
-// decided on the device.
+// decided on the device.  A network whose state fits the SMs' shared memory takes
+// the resident kernel (cmf_resident.cuh) instead.
 
 #include "cmfb200.h"
 #include "cmf_device.cuh"
@@ -627,11 +628,14 @@ int interval_direct(CmfPlan* p, cudaStream_t s, double T, int fixed_n)
 // lists are in the form that the kernel indexes by (k_resident_scan): one tile
 // per SM, as many cells as spread the network over the SMs, and the
 // floodplain rows in shared memory too where they find room.  It is taken
-// wherever it fits, because it was the faster form at every such size.  Through
-// the interval graph and through this kernel: an hour of 4k full physics 854 /
-// 345 us; a day of 60k plain 17.1 / 5.5 ms, of 100k full physics with two
-// statistics 25.4 / 9.6 ms, of 250k full physics 35.3 / 17.1 ms, of 30k full
-// physics in fp64 26.6 / 13.9 ms.
+// wherever it fits and the path ends allow it (above), because it was the faster
+// form there.  Through the interval graph and through this kernel, a single
+// sub-step, an hour and a day (of as many sub-steps as the CFL asks for): 100
+// plain catchments 39 / 15 us, 221 / 64 us, 4.4 / 1.2 ms; 4k full physics 59 / 32
+// us, 1.15 / 0.40 ms, 26.6 / 8.9 ms; 100k plain 43 / 26 us, 0.56 / 0.22 ms, 12.8 /
+// 4.7 ms; 300k plain 51 / 34 us, 1.15 / 0.56 ms, 26.5 / 12.7 ms; 240k full physics
+// 70 / 46 us, 1.29 / 0.60 ms, 29.6 / 13.6 ms; 30k full physics in fp64 57 / 40 us,
+// 1.00 / 0.54 ms, 22.8 / 12.2 ms.
 int plan_resident(CmfPlan* p, const Layout& L)
 {
     p->resident_tiles = 0;

@@ -211,7 +211,10 @@ size_t cmf_view_size(void);
 
 /* ---- plan lifecycle ------------------------------------------------------ */
 /* Bytes of scratch the view needs (Qu fluxes, path sums, budget partials,
- * levee-indexed copies of the levee cells' static fields and marks). */
+ * levee-indexed copies of the levee cells' static fields and marks; for one
+ * member without budget of a size that can fit the SMs' shared memory also the
+ * words that the resident kernel's tiles exchange: 32 bytes per catchment and
+ * 56 per path, twice that with CMF_FEAT_FP64). */
 int cmf_workspace_size(const CmfView* view, size_t* bytes);
 /* Validate the view and bind a plan to its pointers (cmfgpu phys dispatch:
  * BackendRegistry(...).selected binding by parameter name,
@@ -236,8 +239,8 @@ void cmf_plan_destroy(CmfPlan* plan);
  * (CMF_ERR_UNSUPPORTED otherwise, and cmf_stats_attach refuses while it is
  * on); the grid is the device's resident CTAs, or fewer when the network
  * needs fewer.  A barrier wait that outlasts 1 s raises
- * CMF_STATUS_SYNC_TIMEOUT and ends the interval; the state is then undefined.  enable == 0 returns to the
- * interval graph. */
+ * CMF_STATUS_SYNC_TIMEOUT and ends the interval; the state is then undefined.  enable == 0 returns to
+ * the form that the plan takes by itself. */
 int cmf_plan_set_persistent(CmfPlan* plan, int enable);
 /* Tiles of the resident interval kernel that cmf_step_interval takes for this
  * plan: one member without budget whose state fits the SMs' shared memory runs
@@ -353,8 +356,8 @@ int cmf_budget_flush(CmfPlan* plan, void* stream);
  * The reference's `variables_to_save` (scripts/run_daily_bin.py:28, e.g.
  * {"mean": ["total_outflow"], "last": ["river_depth"]}) aggregated by its
  * output layer outside the step.  Here the aggregation is one kernel appended
- * to the sub-step inside the interval graph, so a whole output period runs
- * without a device-to-host copy.  Conventions:
+ * to the sub-step inside the interval graph, or part of the resident kernel, so a
+ * whole output period runs without a device-to-host copy.  Conventions:
  *   MEAN  sum over sub-steps of value * dt, divided at finalize by the sum
  *         of dt of the member (a time average over the output period);
  *   MAX / MIN  over the values after every sub-step (NaN sticks);
