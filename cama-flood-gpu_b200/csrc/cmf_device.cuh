@@ -93,7 +93,7 @@ constexpr int kCtlBarrier = 4;    // [4..5]: arrival counter (u64) of the persis
 constexpr int kCtlAbort = 6;      // set when a wait gave up: every block leaves the interval
 constexpr int kCtlCflMax = 8;     // resident kernel: CFL sub-step count, maximum over the tiles
 constexpr int kCtlEpoch = 9;      // resident kernel: last epoch that exchanged values may carry
-constexpr int kCtlTileMax = 10;   // [10..16]: TileScan of the resident kernel
+constexpr int kCtlTileMax = 10;   // [10..17]: TileScan of the resident kernel
 constexpr int kCtlWords = 32;
 constexpr int kResidentMaxTiles = 256;  // flags of the resident kernel (cmf_resident.cuh)
 constexpr int kHardSubStepCap = 100000;  // bound of the device-side sub-step loop

@@ -672,7 +672,8 @@ int plan_resident(CmfPlan* p, const Layout& L)
     if ((rc = check_cuda(cudaMemcpy(&found, (int*)(ws + L.ctl) + kCtlTileMax, sizeof(found),
                                     cudaMemcpyDeviceToHost))) != CMF_OK)
         return rc;
-    if (found.irregular || found.cell_ends > kResidentCellEnds || found.most.ends > kResidentTileEnds) return CMF_OK;
+    if (found.irregular || found.stray != 0) return CMF_OK;
+    if (found.cell_ends > kResidentCellEnds || found.most.ends > kResidentTileEnds) return CMF_OK;
     a.most = found.most;
     resident_layout(a, real, v.num_flood_levels, v.num_bifurcation_levels, true);
     if (a.bytes > room) resident_layout(a, real, v.num_flood_levels, v.num_bifurcation_levels, false);

@@ -720,6 +720,7 @@ struct TileScan {
     TileCounts most;  // maxima over the tiles
     int irregular;    // not 0: the view's lists are not in the form below
     int cell_ends;    // the most path ends of a cell
+    int stray;        // upstream ranges' cells less the cells that are upstream of one
 };
 
 // TileCounts of every tile (one block each) and the form of the lists that
@@ -727,21 +728,35 @@ struct TileScan {
 // bisection of the levee list and writes its cell's slot, so the list has to be
 // strictly ascending, in range, and exactly the cells flagged as levee cells;
 // a path end elsewhere answers only if its cell is flagged for bifurcation and
-// is the one that the path names.
-// The sub-step kernels ask for neither (levee_slot maps any order).
+// is the one that the path names.  And a cell elsewhere posts to its downstream
+// cell's tile, which waits for all cells of its upstream ranges there: so a mouth
+// flows into itself, every other cell lies in the range of the one it flows into,
+// after it, and the ranges of a tile hold no other cells.
+// The sub-step kernels wait for nothing and ask for none of this.
 template <typename REAL>
 __global__ void __launch_bounds__(256) k_resident_scan(const Dev<REAL> v, int tile)
 {
-    __shared__ int own, dams, levees, bad, lo, hi, cell_ends;
+    __shared__ int own, dams, levees, bad, lo, hi, cell_ends, stray, beyond;
     const int t0 = blockIdx.x * tile, t1 = min(t0 + tile, (int)v.N);
-    if (threadIdx.x == 0) { own = dams = levees = bad = hi = cell_ends = 0; lo = INT32_MAX; }
+    if (threadIdx.x == 0) { own = dams = levees = bad = hi = cell_ends = stray = beyond = 0; lo = INT32_MAX; }
     __syncthreads();
     for (int i = t0 + threadIdx.x; i < t1; i += blockDim.x) {
         const int c0 = v.up[i], c1 = upstream_end(v, (long)i);
         const uint8_t fl = v.flags[i];
+        if (c0 < c1) {
+            if (c0 <= i || c1 > v.N) bad = 1;
+            atomicAdd(&stray, c1 - c0);
+        }
         if (c0 < c1 && c1 > t1) {
             atomicMin(&lo, max(c0, t1));
             atomicMax(&hi, c1);
+            atomicAdd(&beyond, c1 - max(c0, t1));
+        }
+        const int d = v.dn[i];
+        if (((fl & CMF_CELL_MOUTH) != 0) != (d == i)) bad = 1;
+        if (d != i) {
+            if (d < 0 || d >= v.N || i < v.up[d] || i >= upstream_end(v, (long)d)) bad = 1;
+            atomicSub(&stray, 1);
         }
         if ((v.features & CMF_FEAT_RESERVOIR) && (fl & CMF_CELL_RESERVOIR)) atomicAdd(&dams, 1);
         if ((v.features & CMF_FEAT_LEVEE) && (fl & CMF_CELL_LEVEE)) atomicAdd(&levees, 1);
@@ -772,8 +787,9 @@ __global__ void __launch_bounds__(256) k_resident_scan(const Dev<REAL> v, int ti
     atomicMax(most + 2, listed);
     atomicMax(most + 3, dams);
     if (hi > 0) atomicMax(most + 4, hi - lo);
-    if (bad || levees != listed) atomicMax(most + 5, 1);
+    if (bad || levees != listed || (hi > 0 && beyond != hi - lo)) atomicMax(most + 5, 1);
     atomicMax(most + 6, cell_ends);
+    atomicAdd(most + 7, stray);
 }
 
 template <typename REAL, bool RES, bool LEV, bool BIF>

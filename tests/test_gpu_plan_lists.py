@@ -1,6 +1,7 @@
 """Lists of a view in a form that the resident interval kernel cannot index by:
 a levee list that is not ascending, a levee cell that no levee lists, a path end
-in a cell that is not flagged for bifurcation.  The plan leaves such a view to
+in a cell that is not flagged for bifurcation, a mouth whose downstream index is not
+its own.  The plan leaves such a view to
 the interval graph, whose results are those of the same view with the sub-step
 kernels launched one by one; it does the same where a cell or a tile has more
 path ends than the resident kernel is fast with.  Flag bits that the library does
@@ -63,7 +64,21 @@ def test_levees_in_any_order(precision, device):
     _same(_run(plain, net), _run(mixed, net))
 
 
-@pytest.mark.parametrize("change", [_unlisted_levee, _unflagged_path_ends])
+def _mouths_into_another_cell(m):
+    """The downstream index of a mouth, which its flag keeps from being used."""
+    mouths = (m.base.cell_flags & _lib.CELL_MOUTH) != 0
+    m.base.downstream_idx[mouths] = 7
+
+
+def _foreign_upstream_cell(m):
+    """A leaf's upstream range made to hold a cell of another one."""
+    up = m.base.upstream_ptr
+    last = int(up.numel()) - 2
+    up[last] = last - 1
+    up[last + 1] = last
+
+
+@pytest.mark.parametrize("change", [_unlisted_levee, _unflagged_path_ends, _mouths_into_another_cell])
 def test_lists_that_disagree_with_the_flags(change, device):
     net = P.make_network("full", n=5000)
     runs = []
@@ -74,6 +89,15 @@ def test_lists_that_disagree_with_the_flags(change, device):
         assert m.resident_tiles == 0
         runs.append(_run(m, net))
     _same(*runs)
+
+
+def test_upstream_range_with_a_foreign_cell(device):
+    """The plan only: the sub-step kernels would add that cell's flow twice."""
+    m = P.model_for(P.make_network("plain", n=5000))
+    assert m.resident_tiles > 0
+    _foreign_upstream_cell(m)
+    m._rebuild_plan(m.block_size)
+    assert m.resident_tiles == 0
 
 
 def test_undefined_flag_bits_are_ignored(device):
