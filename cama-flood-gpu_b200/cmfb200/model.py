@@ -813,7 +813,11 @@ class CaMaFlood:
     def set_resident(self, on: bool = True) -> None:
         """Whether a network that fits the SMs' shared memory runs its
         intervals in the resident kernel (the default) or through the interval
-        graph; the results are the same."""
+        graph; the results are the same.  One interval is faster in the
+        kernel; four or more large models whose intervals are in flight
+        together on streams of their own share the GPU better through the
+        graph (200 sub-steps of four models of 100k full physics: 10.8 against
+        13.0 ms; of two: 8.9 against 6.5)."""
         _lib.check(_lib.lib().cmf_plan_set_resident(self._plan, 1 if on else 0), "plan_set_resident")
         self.resident = bool(on)
 
