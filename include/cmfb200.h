@@ -221,8 +221,8 @@ int cmf_workspace_size(const CmfView* view, size_t* bytes);
  * cmfgpu/phys/outflow.py:51-60).  Reads the topology, the flags and the lists,
  * which stay as they are while the plan lives: it waits for the device before
  * it does (they may come from any stream) and again before it returns, so it
- * cannot be called inside a stream capture.  With levees, the plan copies each levee
- * cell's floodplain row and (when not member-batched) river height, width
+ * cannot be called inside a stream capture.  With levees, the plan copies each
+ * levee cell's floodplain row and (when not member-batched) river height, width
  * and length into the workspace once, synchronously, and with that shared
  * geometry computes each levee's marks: the storages at which its regimes
  * change (profile filled to the base and to the crown, the river-side wedge)
@@ -239,17 +239,17 @@ void cmf_plan_destroy(CmfPlan* plan);
  * (CMF_ERR_UNSUPPORTED otherwise, and cmf_stats_attach refuses while it is
  * on); the grid is the device's resident CTAs, or fewer when the network
  * needs fewer.  A barrier wait that outlasts 1 s raises
- * CMF_STATUS_SYNC_TIMEOUT and ends the interval; the state is then undefined.  enable == 0 returns to
- * the form that the plan takes by itself. */
+ * CMF_STATUS_SYNC_TIMEOUT and ends the interval; the state is then undefined.
+ * enable == 0 returns to the form that the plan takes by itself. */
 int cmf_plan_set_persistent(CmfPlan* plan, int enable);
 /* Tiles of the resident interval kernel that cmf_step_interval takes for this
  * plan: one member without budget whose state fits the SMs' shared memory runs
- * a whole interval in one cooperative launch after the prologue.  0: the plan takes another form.  Its blocks
- * wait for one another's values; a wait that has polled 2^22 times without
- * success (seconds, where microseconds are usual) raises
- * CMF_STATUS_SYNC_TIMEOUT and ends the interval, and the state and the
- * statistics are then undefined: blocks that need nothing of the one that
- * failed may have written theirs. */
+ * a whole interval in one cooperative launch after the prologue.  0: the plan
+ * takes another form.  The kernel's blocks wait for one another's values; a
+ * wait that has polled 2^22 times without success (seconds, where microseconds
+ * are usual) raises CMF_STATUS_SYNC_TIMEOUT and ends the interval, and the
+ * state and the statistics are then undefined: blocks that need nothing of the
+ * one that failed may have written theirs. */
 int cmf_plan_resident_tiles(const CmfPlan* plan);
 /* enable == 0: such a plan runs its intervals through the interval graph
  * instead, with the same results; enable != 0 (the default) returns to the

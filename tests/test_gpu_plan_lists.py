@@ -1,11 +1,10 @@
 """Lists of a view in a form that the resident interval kernel cannot index by:
 a levee list that is not ascending, a levee cell that no levee lists, a path end
 in a cell that is not flagged for bifurcation, a mouth whose downstream index is not
-its own.  The plan leaves such a view to
-the interval graph, whose results are those of the same view with the sub-step
-kernels launched one by one; it does the same where a cell or a tile has more
-path ends than the resident kernel is fast with.  Flag bits that the library does
-not define change nothing."""
+its own.  The plan leaves such a view to the interval graph, whose results are
+those of the same view with the sub-step kernels launched one by one; it does the
+same where a cell or a tile has more path ends than the resident kernel is fast
+with.  Flag bits that the library does not define change nothing."""
 import numpy as np
 import pytest
 import torch
